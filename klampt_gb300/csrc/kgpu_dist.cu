@@ -60,6 +60,7 @@ struct __align__(16) DistSmem {
   uint32_t jobA[kDJobs], jobB[kDJobs], jobOff[kDJobs + 1];
   uint32_t candA[kDCand], candB[kDCand];
   float candD[kDCand];
+  uint8_t candS[kDCand];  // FP32-separated: the canonical overlap test is not needed
   int pobj[kDPairs];
   int plink[kDPairs];
   float plb[kDPairs];
@@ -117,7 +118,8 @@ __device__ __noinline__ void dist_fk64(DistSmem& S, const KRobotDev& R, double (
 // FP64 finalisation of the pending candidates of pair (l, o): exact squared
 // distances, merged into the running lexicographic best (S.b2, S.bA, S.bB).
 __device__ __noinline__ void flush_cands(DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
-                                         double (*T64)[12], int& fk64, int lane, int l, int ncand, DCnt& cnt)
+                                         double (*T64)[12], int& fk64, int lane, int l, int ncand, float m32,
+                                         DCnt& cnt)
 {
   dist_fk64(S, R, T64, lane, fk64);
   for (int base = 0; base < ncand; base += 32) {
@@ -132,7 +134,16 @@ __device__ __noinline__ void flush_cands(DistSmem& S, const KWorldDev* __restric
       for (int v = 0; v < 3; ++v) kx_xform_point(T64[l], pa + 3 * v, P + 3 * v);
       const double* pb = W->etri64 + 9 * (size_t)tB;
       for (int i = 0; i < 9; ++i) Q[i] = pb[i];
-      d2 = kx_tri_tri_dist2(P, Q, cp, cq);
+      float3 P32[3], Q32[3];
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
+        P32[v] = xform32(S.T[l], make_float3(x.x, x.y, x.z));
+        const float4 y = __ldg(W->etri32 + 3 * (size_t)tB + v);
+        Q32[v] = make_float3(y.x, y.y, y.z);
+      }
+      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[l] + W->eps_env + 2.f * W->eps_extra);
+      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
       oa = W->ltri_orig[tA];
       ob = W->etri_orig[tB];
       cnt.band++;
@@ -317,7 +328,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
         const bool cand = p < total && d32 - e <= lim;
         const unsigned mcand = __ballot_sync(0xffffffffu, cand);
         if (ncand + __popc(mcand) > kDCand) {
-          flush_cands(S, W, R, T64, fk64, lane, l, ncand, cnt);
+          flush_cands(S, W, R, T64, fk64, lane, l, ncand, m32, cnt);
           ncand = 0;
           if (S.b2 < DBL_MAX) m32 = fminf(m32, (float)sqrt(S.b2) * (1.f + 1e-6f));
         }
@@ -326,6 +337,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
           S.candA[r] = (uint32_t)tA;
           S.candB[r] = (uint32_t)tB;
           S.candD[r] = d32 - e;
+          S.candS[r] = d32 > 0.f;
         }
         ncand += __popc(mcand);
         __syncwarp();
@@ -415,20 +427,21 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
       bool ok = false;
       uint32_t a = 0, b = 0;
       float dd = 0.f;
+      uint8_t ss = 0;
       if (k < ncand) {
-        a = S.candA[k]; b = S.candB[k]; dd = S.candD[k];
+        a = S.candA[k]; b = S.candB[k]; dd = S.candD[k]; ss = S.candS[k];
         ok = dd <= lim + 1e-6f;
       }
       __syncwarp();
       const unsigned mk = __ballot_sync(0xffffffffu, ok);
       if (ok) {
         const int r = keep + __popc(mk & lt);
-        S.candA[r] = a; S.candB[r] = b; S.candD[r] = dd;
+        S.candA[r] = a; S.candB[r] = b; S.candD[r] = dd; S.candS[r] = ss;
       }
       keep += __popc(mk);
       __syncwarp();
     }
-    if (keep > 0) flush_cands(S, W, R, T64, fk64, lane, l, keep, cnt);
+    if (keep > 0) flush_cands(S, W, R, T64, fk64, lane, l, keep, m32, cnt);
     if (S.b2 == DBL_MAX) { out.found = 0; return; }
     zero = S.b2 == 0.0;
   }
@@ -942,6 +955,7 @@ struct __align__(16) SelfDistSmem {
   uint32_t jobA[kSDJobs], jobB[kSDJobs], jobOff[kSDJobs + 1];
   uint32_t candA[kSDCand], candB[kSDCand];
   float candD[kSDCand];
+  uint8_t candS[kSDCand];  // FP32-separated: the canonical overlap test is not needed
   double b2, bcp[3], bcq[3];  // best over the pairs so far: squared distance, closest points
   double bd;                   // its distance (the cutoff before any pair is found)
   int bi, bj;
@@ -1009,8 +1023,9 @@ __device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* _
 // of j) over the triangle pairs whose squared distance is below the pair's
 // acceptance bound (the square of the best distance of the earlier pairs)
 __device__ __noinline__ void sd_flush(SelfDistSmem& S, const KWorldDev* __restrict__ W, int lane, int i, int j,
-                                      int ncand, float lim)
+                                      int ncand, float m32)
 {
+  const float lim = m32 * (1.f + 2e-5f) + 1e-6f;
   for (int base = 0; base < ncand; base += 32) {
     const int k = base + lane;
     double d2 = DBL_MAX;
@@ -1025,7 +1040,16 @@ __device__ __noinline__ void sd_flush(SelfDistSmem& S, const KWorldDev* __restri
         kx_xform_point(S.T64[i], pa + 3 * v, P + 3 * v);
         kx_xform_point(S.T64[j], pb + 3 * v, Q + 3 * v);
       }
-      d2 = kx_tri_tri_dist2(P, Q, cp, cq);
+      float3 P32[3], Q32[3];
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
+        P32[v] = xform32(S.T[i], make_float3(x.x, x.y, x.z));
+        const float4 y = __ldg(W->ltri32 + 3 * (size_t)tB + v);
+        Q32[v] = xform32(S.T[j], make_float3(y.x, y.y, y.z));
+      }
+      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[i] + S.delta[j]);
+      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
       oa = W->ltri_orig[tA];
       ob = W->ltri_orig[tB];
     }
@@ -1201,7 +1225,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
             const bool cand = d32 < FLT_MAX && d32 - e <= m32 * (1.f + 2e-5f);
             const unsigned mc = __ballot_sync(0xffffffffu, cand);
             if (ncand + __popc(mc) > kSDCand) {
-              sd_flush(S, W, lane, i, j, ncand, m32 * (1.f + 2e-5f) + 1e-6f);
+              sd_flush(S, W, lane, i, j, ncand, m32);
               ncand = 0;
               if (S.phave) m32 = fminf(m32, (float)sqrt(S.pb2) * (1.f + 1e-6f));
             }
@@ -1210,6 +1234,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
               S.candA[rr] = (uint32_t)tA;
               S.candB[rr] = (uint32_t)tB;
               S.candD[rr] = d32 - e;
+              S.candS[rr] = d32 > 0.f;
             }
             ncand += __popc(mc);
             __syncwarp();
@@ -1281,7 +1306,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
         __syncwarp();
       }
       if (!pc && ncand > 0) {
-        sd_flush(S, W, lane, i, j, ncand, m32 * (1.f + 2e-5f) + 1e-6f);
+        sd_flush(S, W, lane, i, j, ncand, m32);
         if (S.phave) m32 = fminf(m32, (float)sqrt(S.pb2) * (1.f + 1e-6f));
       }
       if (per_pair) {

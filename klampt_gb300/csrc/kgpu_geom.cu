@@ -94,6 +94,7 @@ struct __align__(16) GeomSmem {
   uint32_t jobA[kGJobs], jobB[kGJobs], jobOff[kGJobs + 1];
   uint32_t candA[kGCand], candB[kGCand];
   float candD[kGCand];
+  uint8_t candS[kGCand];  // FP32-separated: the canonical overlap test is not needed
   double pb2, pcp[3], pcq[3];
   int pA, pB, phave;
 };
@@ -170,8 +171,9 @@ __device__ __noinline__ float geom_seed(const GeomDev& GA, const GeomDev& GB, co
 }
 
 __device__ __noinline__ void geom_flush(GeomSmem& S, const GeomDev& GA, const GeomDev& GB, int lane, int ncand,
-                                        float lim)
+                                        float m32)
 {
+  const float lim = m32 * (1.f + 2e-5f) + 1e-6f;
   for (int base = 0; base < ncand; base += 32) {
     const int k = base + lane;
     double d2 = DBL_MAX;
@@ -182,7 +184,11 @@ __device__ __noinline__ void geom_flush(GeomSmem& S, const GeomDev& GA, const Ge
       double P[9], Q[9];
       tri_world64(GA, S.T64[0], tA, P);
       tri_world64(GB, S.T64[1], tB, Q);
-      d2 = kx_tri_tri_dist2(P, Q, cp, cq);
+      float3 P32[3], Q32[3];
+      tri_world32(GA, S.T[0], tA, P32);
+      tri_world32(GB, S.T[1], tB, Q32);
+      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[0] + S.delta[1]);
+      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
       oa = GA.tri_orig[tA];
       ob = GB.tri_orig[tB];
     }
@@ -321,7 +327,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
             const bool cand = d32 < FLT_MAX && d32 - e <= run * (1.f + 2e-5f);
             const unsigned mc = __ballot_sync(0xffffffffu, cand);
             if (ncand + __popc(mc) > kGCand) {
-              geom_flush(S, GA, GB, lane, ncand, run * (1.f + 2e-5f) + 1e-6f);
+              geom_flush(S, GA, GB, lane, ncand, run);
               ncand = 0;
               if (S.phave) run = fminf(run, (float)sqrt(S.pb2) * (1.f + 1e-6f));
             }
@@ -330,6 +336,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
               S.candA[rr] = (uint32_t)tA;
               S.candB[rr] = (uint32_t)tB;
               S.candD[rr] = d32 - e;
+              S.candS[rr] = d32 > 0.f;
             }
             ncand += __popc(mc);
             __syncwarp();
@@ -411,7 +418,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
       if (lane == 0) A.hit[b] = hit ? 1 : 0;
       continue;
     }
-    if (ncand > 0) geom_flush(S, GA, GB, lane, ncand, run * (1.f + 2e-5f) + 1e-6f);
+    if (ncand > 0) geom_flush(S, GA, GB, lane, ncand, run);
     // ---- outputs
     const bool found = S.phave != 0;
     const double dm = found ? kx_sqrt(S.pb2) : 0.0;
