@@ -404,6 +404,7 @@ static __device__ __noinline__ void warp_fk64(const KRobotDev& R, const double* 
   if (lane < nl) kx_joint_local(R.T0P64[lane], R.axis64[lane], R.jtype[lane], q64[lane], T64[lane]);
   __syncwarp();
   if (lane == 0) {
+#pragma unroll 1
     for (int i = 0; i < nl; ++i) {
       int p = R.parents[i];
       if (p < 0) continue;
@@ -413,6 +414,112 @@ static __device__ __noinline__ void warp_fk64(const KRobotDev& R, const double* 
     }
   }
   __syncwarp();
+}
+
+// kx_tri_tri_overlap in a rolled loop: every one of its 17 axes is the cross
+// product of two edges or of a normal and an edge, and the verdict does not
+// depend on their order.  Unrolled it is 60 KB of code at each place it is
+// inlined, run cold between batches of FP32 work: instruction fetches, not the
+// FP64 pipe, then set its time (the distance kernels spent 30-40% of their
+// stalls on them).  Same operations per axis, so the same verdict.
+static __device__ __noinline__ int tri_overlap64(const double* P, const double* Q)
+{
+  // v: p1, p2, q0, q1, q2 relative to P's first vertex; e: edges of P (0-2)
+  // and Q (3-5), their normals (6, 7)
+  double v[5][3], e[8][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    v[0][i] = kx_sub(P[3 + i], P[i]);
+    v[1][i] = kx_sub(P[6 + i], P[i]);
+    v[2][i] = kx_sub(Q[i], P[i]);
+    v[3][i] = kx_sub(Q[3 + i], P[i]);
+    v[4][i] = kx_sub(Q[6 + i], P[i]);
+    e[0][i] = kx_sub(v[0][i], 0.0);
+    e[1][i] = kx_sub(v[1][i], v[0][i]);
+    e[2][i] = kx_sub(0.0, v[1][i]);
+    e[3][i] = kx_sub(v[3][i], v[2][i]);
+    e[4][i] = kx_sub(v[4][i], v[3][i]);
+    e[5][i] = kx_sub(v[2][i], v[4][i]);
+  }
+  kx_cross3(e[0], e[1], e[6]);
+  kx_cross3(e[3], e[4], e[7]);
+#pragma unroll 1
+  for (int k = 0; k < 17; ++k) {
+    // the normals first (the most frequent separators), then edge x edge,
+    // then the in-plane axes
+    const int x = k < 2 ? 3 * k : (k < 11 ? (k - 2) / 3 : (k < 14 ? 6 : 7));
+    const int y = k < 2 ? 3 * k + 1 : (k < 11 ? 3 + (k - 2) % 3 : k - 11);
+    double a[3];
+    kx_cross3(e[x], e[y], a);
+    const double p1 = kx_dot3(a, v[0]), p2 = kx_dot3(a, v[1]);
+    const double q0 = kx_dot3(a, v[2]), q1 = kx_dot3(a, v[3]), q2 = kx_dot3(a, v[4]);
+    const double pmin = fmin(0.0, fmin(p1, p2)), pmax = fmax(0.0, fmax(p1, p2));
+    const double qmin = fmin(q0, fmin(q1, q2)), qmax = fmax(q0, fmax(q1, q2));
+    if (pmax < qmin || qmax < pmin) return 0;
+  }
+  return 1;
+}
+
+// kx_tri_tri_dist2 over the features of `mask` (9 edge-edge, bit 3 i + j;
+// vertices of P against Q, bit 9 + k; vertices of Q against P, bit 12 + k), in
+// its order and arithmetic: equal to it whenever the mask holds the feature
+// that attains the minimum and the triangles are known to be apart.  apart =
+// false: the canonical overlap test decides first, and every feature is
+// evaluated.  Rolled loops, for the reason given at tri_overlap64.
+constexpr unsigned kFeatAll = 0x7fffu;
+constexpr unsigned kFeatFlat = 1u << 15;  // a triangle without area: never taken as apart
+
+static __device__ __noinline__ double tri_dist2_masked64(const double* P, const double* Q, unsigned mask, bool apart,
+                                                         double* cp, double* cq)
+{
+  if (!apart || (mask & kFeatFlat)) {
+    if (tri_overlap64(P, Q)) {
+      for (int i = 0; i < 3; ++i) { cp[i] = P[i]; cq[i] = P[i]; }
+      return 0.0;
+    }
+    mask = kFeatAll;
+  }
+  double p[9], q[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    p[k] = kx_sub(P[k], P[k % 3]);
+    q[k] = kx_sub(Q[k], P[k % 3]);
+  }
+  double best = 1e300, bp[3] = {0, 0, 0}, bq[3] = {0, 0, 0}, c[3], c2[3], d1[3], d2[3];
+#pragma unroll 1
+  for (unsigned m = mask & 0x1ffu; m; m &= m - 1) {
+    const int k = __ffs(m) - 1, i = k / 3, j = k % 3;
+    kx_sub3(p + 3 * (i == 2 ? 0 : i + 1), p + 3 * i, d1);
+    kx_sub3(q + 3 * (j == 2 ? 0 : j + 1), q + 3 * j, d2);
+    const double d = kx_seg_seg(p + 3 * i, d1, q + 3 * j, d2, c, c2);
+    if (d < best) {
+      best = d;
+#pragma unroll
+      for (int t = 0; t < 3; ++t) { bp[t] = c[t]; bq[t] = c2[t]; }
+    }
+  }
+#pragma unroll 1
+  for (unsigned m = (mask & kFeatAll) >> 9; m; m &= m - 1) {
+    const int k = __ffs(m) - 1;
+    const bool ofp = k < 3;  // a vertex of P against Q, or of Q against P
+    const double* x = ofp ? p + 3 * k : q + 3 * (k - 3);
+    const double* t3 = ofp ? q : p;
+    const double d = kx_pt_tri(x, t3, t3 + 3, t3 + 6, c);
+    if (d < best) {
+      best = d;
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        bp[t] = ofp ? x[t] : c[t];
+        bq[t] = ofp ? c[t] : x[t];
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    cp[t] = kx_add(bp[t], P[t]);
+    cq[t] = kx_add(bq[t], P[t]);
+  }
+  return best;
 }
 
 // FP64 re-test of one band pair: link triangle tA of link la against link

@@ -40,27 +40,20 @@
 #include <climits>
 
 #include "kgpu_device.cuh"
-#include "kgpu_dist32.cuh"
+#include "kgpu_pairdist.cuh"
 
 namespace kgpu {
 
 namespace {
 
 constexpr int kDW = 8;         // warps per block
-constexpr int kDStack = 512;   // node-pair stack entries per warp
 constexpr int kDGStack = 512;  // environment-tree stack for gathering objects
-constexpr int kDJobs = 64;     // leaf-pair jobs
-constexpr int kDCand = 64;     // FP64 triangle-pair candidates
 constexpr int kDPairs = 128;   // gathered (link, object) candidates
 constexpr double kSoftK = 30.0;  // pairs beyond m + 30 tau weigh < e^-30 of the leading term
 
 struct __align__(16) DistSmem {
-  uint2 stack[kDStack];
+  PairSmem P;
   uint32_t gstack[kDGStack];
-  uint32_t jobA[kDJobs], jobB[kDJobs], jobOff[kDJobs + 1];
-  uint32_t candA[kDCand], candB[kDCand];
-  float candD[kDCand];
-  uint8_t candS[kDCand];  // FP32-separated: the canonical overlap test is not needed
   int pobj[kDPairs];
   int plink[kDPairs];
   float plb[kDPairs];
@@ -71,10 +64,6 @@ struct __align__(16) DistSmem {
   const float* item_qa;
   const float* item_qb;
   int item_k, item_n;
-  // running exact best of the current pair (FP64 finalisation)
-  double b2;
-  int bA, bB;
-  double bcp[3], bcq[3];
 };
 
 struct DistArgs {
@@ -97,7 +86,8 @@ struct DistArgs {
 };
 
 struct DCnt {
-  unsigned long long pairs = 0, tri = 0, band = 0, nodes = 0;
+  unsigned long long pairs = 0;
+  PairCnt p;  // per lane
 };
 
 __device__ __forceinline__ double item_q64(const DistSmem& S, int lane)
@@ -113,55 +103,6 @@ __device__ __noinline__ void dist_fk64(DistSmem& S, const KRobotDev& R, double (
   __syncwarp();
   warp_fk64(R, S.q64, T64, lane);
   fk64 = 1;
-}
-
-// FP64 finalisation of the pending candidates of pair (l, o): exact squared
-// distances, merged into the running lexicographic best (S.b2, S.bA, S.bB).
-__device__ __noinline__ void flush_cands(DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
-                                         double (*T64)[12], int& fk64, int lane, int l, int ncand, float m32,
-                                         DCnt& cnt)
-{
-  dist_fk64(S, R, T64, lane, fk64);
-  for (int base = 0; base < ncand; base += 32) {
-    const int k = base + lane;
-    double d2 = DBL_MAX;
-    int oa = INT_MAX, ob = INT_MAX;
-    double cp[3] = {0, 0, 0}, cq[3] = {0, 0, 0};
-    if (k < ncand) {
-      const int tA = (int)S.candA[k], tB = (int)S.candB[k];
-      double P[9], Q[9];
-      const double* pa = W->ltri64 + 9 * (size_t)tA;
-      for (int v = 0; v < 3; ++v) kx_xform_point(T64[l], pa + 3 * v, P + 3 * v);
-      const double* pb = W->etri64 + 9 * (size_t)tB;
-      for (int i = 0; i < 9; ++i) Q[i] = pb[i];
-      float3 P32[3], Q32[3];
-#pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
-        P32[v] = xform32(S.T[l], make_float3(x.x, x.y, x.z));
-        const float4 y = __ldg(W->etri32 + 3 * (size_t)tB + v);
-        Q32[v] = make_float3(y.x, y.y, y.z);
-      }
-      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[l] + W->eps_env + 2.f * W->eps_extra);
-      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
-      oa = W->ltri_orig[tA];
-      ob = W->etri_orig[tB];
-      cnt.band++;
-    }
-    int src;
-    double m2 = d2;
-    int ma = oa, mb = ob;
-    warp_lexmin(m2, ma, mb, src, lane);
-    const bool better = m2 < S.b2 || (m2 == S.b2 && (ma < S.bA || (ma == S.bA && mb < S.bB)));
-    __syncwarp();
-    if (better && lane == src) {
-      S.b2 = d2;
-      S.bA = oa;
-      S.bB = ob;
-      for (int i = 0; i < 3; ++i) { S.bcp[i] = cp[i]; S.bcq[i] = cq[i]; }
-    }
-    __syncwarp();
-  }
 }
 
 // An upper bound on the distance between the surfaces of link l and object
@@ -218,241 +159,40 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
                                        PairOut& out, DCnt& cnt, float seed = FLT_MAX)
 {
   cnt.pairs++;
-  const unsigned lt = lanemask_lt();
   const float dl = S.delta[l] + W->eps_extra;
   const float de = W->eps_env + W->eps_extra;
-  const float fb = bound > 0.0 ? (bound < 1e30 ? (float)bound * 1.000001f + 1e-7f : FLT_MAX) : 0.f;
-  float m32 = seed;  // running FP32 minimum (warp-uniform); seed: an upper bound known in advance
-  bool overlap = false;
-  int top = 0, njobs = 0, ncand = 0;
+  // running FP32 upper bound of the minimum: the search bound, or a seed
+  float m32 = fminf(seed, bound > 0.0 ? (bound < 1e30 ? (float)bound * 1.000001f + 1e-7f : FLT_MAX) : 0.f);
   int certA = -1;  // link triangle of the certified contact
+  __syncwarp();    // (the previous pair's results have been read)
   if (lane == 0) {
-    S.b2 = DBL_MAX;
-    S.bA = INT_MAX;
-    S.bB = INT_MAX;
-    S.stack[0] = make_uint2((uint32_t)W->obj_root[o], (uint32_t)R.link_root[l]);
+    S.P.b2 = DBL_MAX;
+    S.P.bA = INT_MAX;
+    S.P.bB = INT_MAX;
+    S.P.have = 0;
   }
-  __syncwarp();
-  top = 1;
   const float* TA = S.T[l];
-#pragma unroll 1
-  while (top > 0 || njobs > 0) {
-    // triangle jobs are tested early (16 at a time): the running minimum they
-    // produce is what prunes the rest of the traversal
-    if (njobs >= 16 || (top == 0 && njobs > 0)) {
-      // ---- triangle pairs, one per lane
-      uint32_t carry = 0;
-      for (int b = 0; b < njobs; b += 32) {
-        const int j = b + lane;
-        uint32_t c = 0;
-        if (j < njobs) c = ((S.jobA[j] >> 28) + 1) * ((S.jobB[j] >> 28) + 1);
-        uint32_t incl = c;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-          if (lane >= off) incl += v;
-        }
-        if (j < njobs) S.jobOff[j] = carry + incl - c;
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      __syncwarp();
-      const uint32_t total = carry;
-#pragma unroll 1
-      for (uint32_t base = 0; base < total && !overlap; base += 32) {
-        const uint32_t p = base + lane;
-        float d32 = FLT_MAX, e = 0.f;
-        bool certain = false;
-        int tA = 0, tB = 0;
-        if (p < total) {
-          int lo = 0, hi = njobs - 1;
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (S.jobOff[mid] <= p) lo = mid; else hi = mid - 1;
-          }
-          const uint32_t r = p - S.jobOff[lo];
-          const uint32_t cb = (S.jobB[lo] >> 28) + 1;
-          tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
-          tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
-          float3 P[3], Q[3];
-#pragma unroll
-          for (int v = 0; v < 3; ++v) {
-            const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
-            P[v] = xform32(TA, make_float3(x.x, x.y, x.z));
-            const float4 y = __ldg(W->etri32 + 3 * (size_t)tB + v);
-            Q[v] = make_float3(y.x, y.y, y.z);
-          }
-          float3 lo3 = P[0], hi3 = P[0];
-#pragma unroll
-          for (int k = 1; k < 6; ++k) {
-            const float3 v = k < 3 ? P[k] : Q[k - 3];
-            lo3 = make_float3(fminf(lo3.x, v.x), fminf(lo3.y, v.y), fminf(lo3.z, v.z));
-            hi3 = make_float3(fmaxf(hi3.x, v.x), fmaxf(hi3.y, v.y), fmaxf(hi3.z, v.z));
-          }
-          const float span = fmaxf(fmaxf(hi3.x - lo3.x, hi3.y - lo3.y), hi3.z - lo3.z);
-          e = dl + de + 128.f * kU * span + 1e-8f;
-          // triangle-box lower bound: skip the full distance when it cannot
-          // be a candidate
-          float3 pl = P[0], ph = P[0], ql = Q[0], qh = Q[0];
-#pragma unroll
-          for (int k = 1; k < 3; ++k) {
-            pl = make_float3(fminf(pl.x, P[k].x), fminf(pl.y, P[k].y), fminf(pl.z, P[k].z));
-            ph = make_float3(fmaxf(ph.x, P[k].x), fmaxf(ph.y, P[k].y), fmaxf(ph.z, P[k].z));
-            ql = make_float3(fminf(ql.x, Q[k].x), fminf(ql.y, Q[k].y), fminf(ql.z, Q[k].z));
-            qh = make_float3(fmaxf(qh.x, Q[k].x), fmaxf(qh.y, Q[k].y), fmaxf(qh.z, Q[k].z));
-          }
-          const float gx = fmaxf(0.f, fmaxf(ql.x - ph.x, pl.x - qh.x));
-          const float gy = fmaxf(0.f, fmaxf(ql.y - ph.y, pl.y - qh.y));
-          const float gz = fmaxf(0.f, fmaxf(ql.z - ph.z, pl.z - qh.z));
-          const float blb = sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU);
-          const float skip = fminf(m32 * (1.f + 2e-5f) + 2.f * e, fb + e);
-          if (blb - e > skip || tri_axis_lb32(P, Q, span) - e > skip) {
-            d32 = FLT_MAX;  // not a candidate (and no better than the running minimum)
-          } else if (!tri_separated32(P, Q, dl + de, 0.f)) {
-            d32 = 0.f;
-            certain = tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], fmaxf(dl, de));
-          } else {
-            d32 = sqrtf(tri_dist2_32(P, Q));
-          }
-          cnt.tri++;
-        }
-        const unsigned mc = __ballot_sync(0xffffffffu, certain);
-        if (mc) {
-          overlap = true;
-          const int src = __ffs(mc) - 1;
-          certA = __shfl_sync(0xffffffffu, tA, src);
-          break;
-        }
-        m32 = fminf(m32, warp_min(d32));
-        const float emax = warp_min(-e) * -1.f;  // largest band in this batch
-        const float lim = fminf(m32 * (1.f + 2e-5f) + 2.f * emax, fb + emax);
-        const bool cand = p < total && d32 - e <= lim;
-        const unsigned mcand = __ballot_sync(0xffffffffu, cand);
-        if (ncand + __popc(mcand) > kDCand) {
-          flush_cands(S, W, R, T64, fk64, lane, l, ncand, m32, cnt);
-          ncand = 0;
-          if (S.b2 < DBL_MAX) m32 = fminf(m32, (float)sqrt(S.b2) * (1.f + 1e-6f));
-        }
-        if (cand) {
-          const int r = ncand + __popc(mcand & lt);
-          S.candA[r] = (uint32_t)tA;
-          S.candB[r] = (uint32_t)tB;
-          S.candD[r] = d32 - e;
-          S.candS[r] = d32 > 0.f;
-        }
-        ncand += __popc(mcand);
-        __syncwarp();
-      }
-      njobs = 0;
-      if (overlap) break;
-      continue;
-    }
-    // ---- node pairs.  A batch of n pops grows the stack by at most n; near
-    // the capacity the batch narrows down to plain depth-first order (one
-    // pair), whose growth is bounded by the depth of the two trees, so a
-    // wide front (a link deep inside an obstacle, where no box is pruned)
-    // does not overflow the stack
-    const int n = min(min(top, 32), max(1, kDStack - 64 - top));
-    const bool have = lane < n;
-    uint2 en = make_uint2(0, 0);
-    if (have) en = S.stack[top - 1 - lane];
-    __syncwarp();
-    top -= n;
-    int outcome = 0;
-    uint2 c0 = make_uint2(0, 0), c1 = make_uint2(0, 0);
-    uint32_t jA = 0, jB = 0;
-    cnt.nodes += have ? 1 : 0;
-    if (have) {
-      const int nodeB = (int)en.x, nodeA = (int)en.y;
-      const KNode na = W->lnodes[nodeA];
-      const KNode nb = W->enodes[nodeB];
-      const Box32 A = xform_box(TA, na.a, na.b);
-      const float slack = 4.f * kU * (fabsf(A.c.x) + fabsf(A.c.y) + fabsf(A.c.z) + 1.f);
-      const float lb_box = box_dist32(A, make_float3(nb.a.x, nb.a.y, nb.a.z), make_float3(nb.b.x, nb.b.y, nb.b.z)) -
-                           (dl + de) * 1.7321f - slack;
-      // the rotation-invariant sphere about the node centre is tighter than the
-      // world box of a rotated node in most directions
-      const float gx = fmaxf(0.f, fabsf(A.c.x - nb.a.x) - nb.b.x);
-      const float gy = fmaxf(0.f, fabsf(A.c.y - nb.a.y) - nb.b.y);
-      const float gz = fmaxf(0.f, fabsf(A.c.z - nb.a.z) - nb.b.z);
-      const float lb_sph = sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU) - __ldg(W->lnode_r + nodeA) -
-                           (dl + de) * 1.7321f - slack;
-      const float lb = fmaxf(lb_box, lb_sph);
-      const float lim = fminf(m32 * (1.f + 2e-5f) + 3.f * (dl + de) + 1e-5f, fb + 2.f * (dl + de) + 1e-5f);
-      if (lb <= lim) {
-        const int cntA = f2i(na.b.w), cntB = f2i(nb.b.w);
-        const int ia = f2i(na.a.w), ib = f2i(nb.a.w);
-        if (cntA > 0 && cntB > 0) {
-          outcome = 2;
-          jA = (uint32_t)ia | ((uint32_t)(cntA - 1) << 28);
-          jB = (uint32_t)ib | ((uint32_t)(cntB - 1) << 28);
-        } else {
-          outcome = 1;
-          const bool splitB = cntA > 0 || (cntB == 0 && (nb.b.x + nb.b.y + nb.b.z) > (na.b.x + na.b.y + na.b.z));
-          if (splitB) { c0 = make_uint2((uint32_t)ib, (uint32_t)nodeA); c1 = make_uint2((uint32_t)ib + 1, (uint32_t)nodeA); }
-          else { c0 = make_uint2((uint32_t)nodeB, (uint32_t)ia); c1 = make_uint2((uint32_t)nodeB, (uint32_t)ia + 1); }
-        }
-      }
-    }
-    const unsigned m1 = __ballot_sync(0xffffffffu, outcome == 1);
-    const unsigned m2 = __ballot_sync(0xffffffffu, outcome == 2);
-    if (top + 2 * __popc(m1) > kDStack) {
-      // stack would overflow: the pair is evaluated conservatively by giving up
-      // pruning precision is not an option, so flag and stop
-      if (lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
-      out.found = 0;
-      return;
-    }
-    if (outcome == 1) {
-      const int r = top + 2 * __popc(m1 & lt);
-      S.stack[r] = c1;
-      S.stack[r + 1] = c0;
-    } else if (outcome == 2) {
-      const int r = njobs + __popc(m2 & lt);
-      S.jobA[r] = jA;
-      S.jobB[r] = jB;
-    }
-    top += 2 * __popc(m1);
-    njobs += __popc(m2);
-    __syncwarp();
+  const MeshView A = {W->lnodes, W->lnode_r, W->ltri32, W->ltri64, W->ltri_orig};
+  const MeshView B = {W->enodes, nullptr, W->etri32, W->etri64, W->etri_orig};
+  const int r = pair_distance<true, true>(S.P, A, B, R.link_root[l], W->obj_root[o], TA, nullptr, T64[l], nullptr,
+                                          dl + de, m32, certA, lane, cnt.p,
+                                          [&] { dist_fk64(S, R, T64, lane, fk64); });
+  if (r == 2) {
+    if (lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
+    out.found = 0;
+    return;
   }
-
-  // ---- unsigned distance: exact zero (certified contact) or FP64 finalisation
-  bool zero = overlap;
-  if (!overlap) {
-    // drop stale candidates, then finalise
-    const float lim = fminf(m32 * (1.f + 2e-5f), fb);
-    int keep = 0;
-    for (int base = 0; base < ncand; base += 32) {
-      const int k = base + lane;
-      bool ok = false;
-      uint32_t a = 0, b = 0;
-      float dd = 0.f;
-      uint8_t ss = 0;
-      if (k < ncand) {
-        a = S.candA[k]; b = S.candB[k]; dd = S.candD[k]; ss = S.candS[k];
-        ok = dd <= lim + 1e-6f;
-      }
-      __syncwarp();
-      const unsigned mk = __ballot_sync(0xffffffffu, ok);
-      if (ok) {
-        const int r = keep + __popc(mk & lt);
-        S.candA[r] = a; S.candB[r] = b; S.candD[r] = dd; S.candS[r] = ss;
-      }
-      keep += __popc(mk);
-      __syncwarp();
-    }
-    if (keep > 0) flush_cands(S, W, R, T64, fk64, lane, l, keep, m32, cnt);
-    if (S.b2 == DBL_MAX) { out.found = 0; return; }
-    zero = S.b2 == 0.0;
-  }
+  if (r == 0 && !S.P.have) { out.found = 0; return; }
+  // unsigned distance: exact zero (certified contact) or the FP64 minimum
+  const bool zero = r == 1 || S.P.b2 == 0.0;
   if (!zero) {
-    const double d = kx_sqrt(S.b2);
+    const double d = kx_sqrt(S.P.b2);
     out.found = d < bound;
     out.d = d;
     for (int i = 0; i < 3; ++i) {
-      out.cp[i] = S.bcp[i];
-      out.cq[i] = S.bcq[i];
-      out.dir[i] = (float)((S.bcp[i] - S.bcq[i]) / d);
+      out.cp[i] = S.P.bcp[i];
+      out.cq[i] = S.P.bcq[i];
+      out.dir[i] = (float)((S.P.bcp[i] - S.P.bcq[i]) / d);
     }
     return;
   }
@@ -477,6 +217,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
     int cv0 = 0, cv1 = 0, nc = 0;
     float cd0 = 0.f, cd1 = 0.f;
     bool rescan = false;
+#pragma unroll 1
     for (int v = lane; v < vc; v += 32) {
       const float4 x = __ldg(W->lvert32 + vf + v);
       const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
@@ -487,6 +228,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
       // (or outside the band): its final minimum can only be lower
       const float stop = fmaxf(lmax, -ed);
       float dmin = FLT_MAX;
+#pragma unroll 1
       for (int f = ff; f < ff + fc && dmin > stop; ++f) {
         const float4 pl = __ldg(W->eface32 + f);
         dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
@@ -518,6 +260,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
           return;
         const float stop = fmaxf(gmax - 2.f * ed, -ed);
         float dmin = FLT_MAX;
+#pragma unroll 1
         for (int f = ff; f < ff + fc && dmin >= stop; ++f) {
           const float4 pl = __ldg(W->eface32 + f);
           dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
@@ -527,6 +270,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
         kx_xform_point(T64[l], W->lvert64 + 3 * (size_t)(vf + v), w64);
         double dm = DBL_MAX;
         int fm = -1, fo = INT_MAX;
+#pragma unroll 1
         for (int f = ff; f < ff + fc; ++f) {
           const double* pl = W->eface64 + 4 * (size_t)f;
           const double dep = kx_sub(pl[3], kx_dot3(pl, w64));
@@ -536,6 +280,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
         if (dm > bd || (dm == bd && dm > 0.0 && v < bv)) { bd = dm; bv = v; bf = fm; }
       };
       if (rescan) {
+#pragma unroll 1
         for (int v = lane; v < vc; v += 32) depth64(v);
       } else {
         if (nc >= 1 && cd0 >= gmax - 2.f * ed) depth64(cv0);
@@ -878,7 +623,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     }
   }
   // counters: pairs are counted once per warp (lane 0), the rest per lane
-  unsigned long long nd = cnt.nodes, tp = cnt.tri, bd = cnt.band;
+  unsigned long long nd = cnt.p.nodes, tp = cnt.p.tri, bd = cnt.p.fp64;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     nd += __shfl_down_sync(0xffffffffu, nd, o);
@@ -938,10 +683,6 @@ __global__ void k_softmin_final(const double* wsum, const double* m, int T, int 
 // transforms.  One warp per configuration: FP32 traversal of each pair with
 // conservative pruning against the running upper bound of the minimum,
 // triangle pairs within the error band finalised in canonical FP64.
-constexpr int kSDStack = 512;
-constexpr int kSDJobs = 64;
-constexpr int kSDCand = 128;
-
 struct __align__(16) SelfDistSmem;
 __device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                              int lane, int i, int j);
@@ -951,16 +692,10 @@ struct __align__(16) SelfDistSmem {
   float delta[kMaxLinks];
   double T64[kMaxLinks][12];
   double q64[kMaxLinks];
-  uint2 stack[kSDStack];
-  uint32_t jobA[kSDJobs], jobB[kSDJobs], jobOff[kSDJobs + 1];
-  uint32_t candA[kSDCand], candB[kSDCand];
-  float candD[kSDCand];
-  uint8_t candS[kSDCand];  // FP32-separated: the canonical overlap test is not needed
+  PairSmem P;                  // the current pair; P.b2 starts at the acceptance bound
   double b2, bcp[3], bcq[3];  // best over the pairs so far: squared distance, closest points
   double bd;                   // its distance (the cutoff before any pair is found)
   int bi, bj;
-  double pb2, pcp[3], pcq[3];  // best of the current pair (pb2 starts at the acceptance bound)
-  int pA, pB, phave;
 };
 
 struct SelfDistArgs {
@@ -1018,67 +753,13 @@ __device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* _
   return sqrtf(bo) * (1.f + 1e-5f) + 2.f * (S.delta[i] + S.delta[j]) + 1e-6f;
 }
 
-// FP64 finalisation of candidates of pair (i, j), merged into the pair's
-// best: the lexicographic minimum (squared distance, triangle of i, triangle
-// of j) over the triangle pairs whose squared distance is below the pair's
-// acceptance bound (the square of the best distance of the earlier pairs)
-__device__ __noinline__ void sd_flush(SelfDistSmem& S, const KWorldDev* __restrict__ W, int lane, int i, int j,
-                                      int ncand, float m32)
-{
-  const float lim = m32 * (1.f + 2e-5f) + 1e-6f;
-  for (int base = 0; base < ncand; base += 32) {
-    const int k = base + lane;
-    double d2 = DBL_MAX;
-    int oa = INT_MAX, ob = INT_MAX;
-    double cp[3] = {0, 0, 0}, cq[3] = {0, 0, 0};
-    if (k < ncand && S.candD[k] <= lim) {
-      const int tA = (int)S.candA[k], tB = (int)S.candB[k];
-      double P[9], Q[9];
-      const double* pa = W->ltri64 + 9 * (size_t)tA;
-      const double* pb = W->ltri64 + 9 * (size_t)tB;
-      for (int v = 0; v < 3; ++v) {
-        kx_xform_point(S.T64[i], pa + 3 * v, P + 3 * v);
-        kx_xform_point(S.T64[j], pb + 3 * v, Q + 3 * v);
-      }
-      float3 P32[3], Q32[3];
-#pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
-        P32[v] = xform32(S.T[i], make_float3(x.x, x.y, x.z));
-        const float4 y = __ldg(W->ltri32 + 3 * (size_t)tB + v);
-        Q32[v] = xform32(S.T[j], make_float3(y.x, y.y, y.z));
-      }
-      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[i] + S.delta[j]);
-      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
-      oa = W->ltri_orig[tA];
-      ob = W->ltri_orig[tB];
-    }
-    int src;
-    double m2 = d2;
-    int ma = oa, mb = ob;
-    warp_lexmin(m2, ma, mb, src, lane);
-    // below the acceptance bound, or equal to the pair's best with smaller
-    // triangles
-    const bool better = S.phave ? (m2 < S.pb2 || (m2 == S.pb2 && (ma < S.pA || (ma == S.pA && mb < S.pB))))
-                                : m2 < S.pb2;
-    __syncwarp();
-    if (m2 < DBL_MAX && better && lane == src) {
-      S.pb2 = d2;
-      S.pA = oa;
-      S.pB = ob;
-      S.phave = 1;
-      for (int c = 0; c < 3; ++c) { S.pcp[c] = cp[c]; S.pcq[c] = cq[c]; }
-    }
-    __syncwarp();
-  }
-}
-
 __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   SelfDistSmem& S = reinterpret_cast<SelfDistSmem*>(smem_raw)[warp];
-  const unsigned lt = lanemask_lt();
+  const MeshView M = {W->lnodes, W->lnode_r, W->ltri32, W->ltri64, W->ltri_orig};
+  PairCnt cnt;
   const KRobotDev& R = W->robots[A.robot];
   const int nl = R.nlinks;
   const float fcut = A.cutoff < 1e30 ? (float)A.cutoff * 1.000001f + 1e-7f : FLT_MAX;
@@ -1128,10 +809,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
         j = (qw >> 8) & 0xff;
       }
       if (R.link_root[i] < 0 || R.link_root[j] < 0) continue;
-      const float* TA = S.T[i];
-      const float* TB = S.T[j];
       const float dd = S.delta[i] + S.delta[j];
-      int top = 1, njobs = 0, ncand = 0;
       bool pc = false;  // certified contact of this pair
       if (per_pair) m32 = fcut;  // every pair on its own
       // a pair without a running bound to prune with (the first, or every
@@ -1141,192 +819,44 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
       if (m32 >= fcut) m32 = fminf(m32, link_pair_seed(S, W, R, lane, i, j));
       if (lane == 0) {
         if (per_pair) S.bd = A.cutoff;
-        S.stack[0] = make_uint2((uint32_t)R.link_root[i], (uint32_t)R.link_root[j]);
         const double bb = kx_mul(S.bd, S.bd);
-        S.pb2 = bb > 1e-300 ? bb : 1e-300;
-        S.pA = S.pB = INT_MAX;
-        S.phave = 0;
+        S.P.b2 = bb > 1e-300 ? bb : 1e-300;
+        S.P.bA = S.P.bB = INT_MAX;
+        S.P.have = 0;
       }
-      __syncwarp();
-#pragma unroll 1
-      while ((top > 0 || njobs > 0) && !pc) {
-        if (njobs >= 16 || (top == 0 && njobs > 0)) {
-          // ---- triangle pairs, one per lane
-          uint32_t carry = 0;
-          for (int bb = 0; bb < njobs; bb += 32) {
-            const int jj = bb + lane;
-            uint32_t c = 0;
-            if (jj < njobs) c = ((S.jobA[jj] >> 28) + 1) * ((S.jobB[jj] >> 28) + 1);
-            uint32_t incl = c;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-              const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-              if (lane >= off) incl += v;
-            }
-            if (jj < njobs) S.jobOff[jj] = carry + incl - c;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-          }
-          __syncwarp();
-          const uint32_t total = carry;
-#pragma unroll 1
-          for (uint32_t base = 0; base < total; base += 32) {
-            const uint32_t p = base + lane;
-            float d32 = FLT_MAX, e = 0.f;
-            int tA = 0, tB = 0;
-            bool certain = false;
-            if (p < total) {
-              int lo = 0, hi = njobs - 1;
-              while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (S.jobOff[mid] <= p) lo = mid; else hi = mid - 1;
-              }
-              const uint32_t r = p - S.jobOff[lo];
-              const uint32_t cb = (S.jobB[lo] >> 28) + 1;
-              tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
-              tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
-              float3 P[3], Q[3];
-#pragma unroll
-              for (int v = 0; v < 3; ++v) {
-                const float4 x = __ldg(W->ltri32 + 3 * (size_t)tA + v);
-                P[v] = xform32(TA, make_float3(x.x, x.y, x.z));
-                const float4 y = __ldg(W->ltri32 + 3 * (size_t)tB + v);
-                Q[v] = xform32(TB, make_float3(y.x, y.y, y.z));
-              }
-              float3 lo3 = P[0], hi3 = P[0];
-#pragma unroll
-              for (int k = 1; k < 6; ++k) {
-                const float3 v = k < 3 ? P[k] : Q[k - 3];
-                lo3 = make_float3(fminf(lo3.x, v.x), fminf(lo3.y, v.y), fminf(lo3.z, v.z));
-                hi3 = make_float3(fmaxf(hi3.x, v.x), fmaxf(hi3.y, v.y), fmaxf(hi3.z, v.z));
-              }
-              const float span = fmaxf(fmaxf(hi3.x - lo3.x, hi3.y - lo3.y), hi3.z - lo3.z);
-              e = dd + 128.f * kU * span + 1e-8f;
-              if (tri_axis_lb32(P, Q, span) - e > m32 * (1.f + 2e-5f) + 2.f * e) {
-                d32 = FLT_MAX;  // cannot be a candidate
-              } else if (!tri_separated32(P, Q, dd, 0.f)) {
-                d32 = 0.f;
-                certain = tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd);
-              } else {
-                d32 = sqrtf(tri_dist2_32(P, Q));
-              }
-            }
-            if (__any_sync(0xffffffffu, certain)) {
-              pc = true;  // distance 0: no later pair can be smaller
-              if (lane == 0 && !per_pair) {
-                S.b2 = 0.0;
-                S.bd = 0.0;
-                S.bi = i;
-                S.bj = j;
-              }
-              __syncwarp();
-              break;
-            }
-            m32 = fminf(m32, warp_min(d32 < FLT_MAX ? d32 + e : FLT_MAX));
-            const bool cand = d32 < FLT_MAX && d32 - e <= m32 * (1.f + 2e-5f);
-            const unsigned mc = __ballot_sync(0xffffffffu, cand);
-            if (ncand + __popc(mc) > kSDCand) {
-              sd_flush(S, W, lane, i, j, ncand, m32);
-              ncand = 0;
-              if (S.phave) m32 = fminf(m32, (float)sqrt(S.pb2) * (1.f + 1e-6f));
-            }
-            if (cand) {
-              const int rr = ncand + __popc(mc & lt);
-              S.candA[rr] = (uint32_t)tA;
-              S.candB[rr] = (uint32_t)tB;
-              S.candD[rr] = d32 - e;
-              S.candS[rr] = d32 > 0.f;
-            }
-            ncand += __popc(mc);
-            __syncwarp();
-          }
-          njobs = 0;
-          continue;
+      int certA = -1;
+      const int r = pair_distance<false, true>(S.P, M, M, R.link_root[i], R.link_root[j], S.T[i], S.T[j], S.T64[i],
+                                               S.T64[j], dd, m32, certA, lane, cnt, [] {});
+      if (r == 2) {
+        if (lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
+      } else if (r == 1) {
+        pc = true;  // distance 0: no later pair can be smaller
+        if (lane == 0 && !per_pair) {
+          S.b2 = 0.0;
+          S.bd = 0.0;
+          S.bi = i;
+          S.bj = j;
         }
-        // ---- node pairs; near the stack capacity the batch narrows to
-        // depth-first order, whose growth is bounded by the trees' depth
-        const int n = min(min(top, 32), max(1, kSDStack - 64 - top));
-        const bool have = lane < n;
-        uint2 en = make_uint2(0, 0);
-        if (have) en = S.stack[top - 1 - lane];
         __syncwarp();
-        top -= n;
-        int outcome = 0;
-        uint2 c0 = make_uint2(0, 0), c1 = make_uint2(0, 0);
-        uint32_t jA = 0, jB = 0;
-        if (have) {
-          const int nodeA = (int)en.x, nodeB = (int)en.y;
-          const KNode na = W->lnodes[nodeA];
-          const KNode nb = W->lnodes[nodeB];
-          const Box32 BA = xform_box(TA, na.a, na.b);
-          const Box32 BB = xform_box(TB, nb.a, nb.b);
-          const float slack = 4.f * kU * (fabsf(BA.c.x) + fabsf(BA.c.y) + fabsf(BA.c.z) + fabsf(BB.c.x) +
-                                          fabsf(BB.c.y) + fabsf(BB.c.z) + 1.f);
-          const float lb_box = box_dist32(BA, BB.c, BB.h) - dd * 1.7321f - slack;
-          const float cx = BA.c.x - BB.c.x, cy = BA.c.y - BB.c.y, cz = BA.c.z - BB.c.z;
-          const float lb_sph = sqrtf(cx * cx + cy * cy + cz * cz) * (1.f - 4.f * kU) - __ldg(W->lnode_r + nodeA) -
-                               __ldg(W->lnode_r + nodeB) - dd * 1.7321f - slack;
-          const float lb = fmaxf(lb_box, lb_sph);
-          if (lb <= m32 * (1.f + 2e-5f) + 3.f * dd + 1e-5f) {
-            const int cntA = f2i(na.b.w), cntB = f2i(nb.b.w);
-            const int ia = f2i(na.a.w), ib = f2i(nb.a.w);
-            if (cntA > 0 && cntB > 0) {
-              outcome = 2;
-              jA = (uint32_t)ia | ((uint32_t)(cntA - 1) << 28);
-              jB = (uint32_t)ib | ((uint32_t)(cntB - 1) << 28);
-            } else {
-              outcome = 1;
-              const bool splitB = cntA > 0 || (cntB == 0 && (nb.b.x + nb.b.y + nb.b.z) > (na.b.x + na.b.y + na.b.z));
-              if (splitB) { c0 = make_uint2((uint32_t)nodeA, (uint32_t)ib); c1 = make_uint2((uint32_t)nodeA, (uint32_t)ib + 1); }
-              else { c0 = make_uint2((uint32_t)ia, (uint32_t)nodeB); c1 = make_uint2((uint32_t)ia + 1, (uint32_t)nodeB); }
-            }
-          }
-        }
-        const unsigned m1 = __ballot_sync(0xffffffffu, outcome == 1);
-        const unsigned m2 = __ballot_sync(0xffffffffu, outcome == 2);
-        if (top + 2 * __popc(m1) > kSDStack) {
-          // cannot happen with the narrowing above (growth bounded by the
-          // trees' depth); checked so that an error is reported, not hidden
-          if (lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
-          top = 0;
-          njobs = 0;
-          ncand = 0;
-          break;
-        }
-        if (outcome == 1) {
-          const int rr = top + 2 * __popc(m1 & lt);
-          S.stack[rr] = c1;
-          S.stack[rr + 1] = c0;
-        } else if (outcome == 2) {
-          const int rr = njobs + __popc(m2 & lt);
-          S.jobA[rr] = jA;
-          S.jobB[rr] = jB;
-        }
-        top += 2 * __popc(m1);
-        njobs += __popc(m2);
-        __syncwarp();
-      }
-      if (!pc && ncand > 0) {
-        sd_flush(S, W, lane, i, j, ncand, m32);
-        if (S.phave) m32 = fminf(m32, (float)sqrt(S.pb2) * (1.f + 1e-6f));
       }
       if (per_pair) {
         if (lane == 0)
           A.dpair[(size_t)b * npair + i * nl - i * (i + 1) / 2 + (j - i - 1)] =
-              pc ? 0.0 : (S.phave ? kx_sqrt(S.pb2) : A.cutoff);
+              pc ? 0.0 : (S.P.have ? kx_sqrt(S.P.b2) : A.cutoff);
         __syncwarp();
         continue;
       }
       // the pair replaces the best only with a strictly smaller distance
-      if (!pc && S.phave) {
-        const double dp = kx_sqrt(S.pb2);
+      if (!pc && S.P.have) {
+        const double dp = kx_sqrt(S.P.b2);
         if (dp < S.bd) {
           __syncwarp();
           if (lane == 0) {
-            S.b2 = S.pb2;
+            S.b2 = S.P.b2;
             S.bd = dp;
             S.bi = i;
             S.bj = j;
-            for (int c = 0; c < 3; ++c) { S.bcp[c] = S.pcp[c]; S.bcq[c] = S.pcq[c]; }
+            for (int c = 0; c < 3; ++c) { S.bcp[c] = S.P.bcp[c]; S.bcq[c] = S.P.bcq[c]; }
           }
         }
       }

@@ -123,7 +123,7 @@ static __device__ float tri_dist2_32(const float3* P, const float3* Q)
 // ---- which features the canonical FP64 distance still has to look at --------
 // kx_tri_tri_dist2 is the minimum over 15 features (9 edge-edge, 3 vertices of
 // P against Q, 3 of Q against P; bit 3 i + j, 9 + k, 12 + k), taken in that
-// order with strict comparisons.  An FP64 operation occupies the SM for 19
+// order with strict comparisons (tri_dist2_masked64).  An FP64 operation occupies the SM for 19
 // cycles per warp whatever the number of active lanes, and all 15 features
 // plus the 17 overlap axes are ~2,300 of them; in FP32 the features are a few
 // hundred full-rate instructions.  Measured (before -> after): 8,192 humanoid
@@ -140,11 +140,9 @@ static __device__ float tri_dist2_32(const float3* P, const float3* Q)
 // of |n|^2 >= 0.01 L^4 (L its longest edge) the foot moves by at most
 // min(L, 6u p^2 / (0.01 L)), p <= span, within 2e-5 span^2 as well.  thr2
 // includes 2e-5 span^2; features worse conditioned than that are always kept.
-// kFeatFlat: a triangle without area, for which the canonical overlap test
-// can report a contact of triangles that are apart (its axes vanish); such a
+// kFeatFlat is set when a triangle has no area: the canonical overlap test can
+// report a contact of such triangles that are apart (its axes vanish), so the
 // pair is left to the whole canonical function.
-constexpr unsigned kFeatFlat = 1u << 15;
-
 static __device__ __noinline__ unsigned tri_feature_mask32(const float3* P, const float3* Q, float thr2)
 {
   unsigned mask = 0;
@@ -190,59 +188,6 @@ __device__ __forceinline__ float feature_thr2(const float3* P, const float3* Q, 
   const float span = fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z);
   const float thr = m32 * (1.f + 2e-5f) + 2.f * (place + 128.f * kU * span) + 1e-6f;
   return thr * thr * (1.f + 1e-5f) + 2e-5f * span * span;  // (FLT_MAX bounds overflow to inf: every feature kept)
-}
-
-// kx_tri_tri_dist2 over the features of `mask` only, in the same order and
-// arithmetic: equal to it whenever the mask holds the feature that attains
-// the minimum and the triangles are known to be apart.  apart = false: the
-// canonical overlap test decides first, and every feature is evaluated.
-static __device__ __noinline__ double tri_dist2_masked64(const double* P, const double* Q, unsigned mask, bool apart,
-                                                         double* cp, double* cq)
-{
-  if (!apart || (mask & kFeatFlat)) {
-    if (kx_tri_tri_overlap(P, Q)) {
-      for (int i = 0; i < 3; ++i) { cp[i] = P[i]; cq[i] = P[i]; }
-      return 0.0;
-    }
-    mask = 0x7fffu;
-  }
-  double p[9], q[9];
-  for (int k = 0; k < 9; ++k) {
-    p[k] = kx_sub(P[k], P[k % 3]);
-    q[k] = kx_sub(Q[k], P[k % 3]);
-  }
-  double best = 1e300, bp[3] = {0, 0, 0}, bq[3] = {0, 0, 0}, c[3], c2[3], d1[3], d2[3];
-#pragma unroll 1
-  for (unsigned m = mask & 0x1ffu; m; m &= m - 1) {
-    const int k = __ffs(m) - 1, i = k / 3, j = k % 3;
-    kx_sub3(p + 3 * (i == 2 ? 0 : i + 1), p + 3 * i, d1);
-    kx_sub3(q + 3 * (j == 2 ? 0 : j + 1), q + 3 * j, d2);
-    const double d = kx_seg_seg(p + 3 * i, d1, q + 3 * j, d2, c, c2);
-    if (d < best) {
-      best = d;
-      for (int t = 0; t < 3; ++t) { bp[t] = c[t]; bq[t] = c2[t]; }
-    }
-  }
-#pragma unroll 1
-  for (unsigned m = (mask & 0x7fffu) >> 9; m; m &= m - 1) {
-    const int k = __ffs(m) - 1;
-    const bool ofp = k < 3;  // a vertex of P against Q, or of Q against P
-    const double* x = ofp ? p + 3 * k : q + 3 * (k - 3);
-    const double* t3 = ofp ? q : p;
-    const double d = kx_pt_tri(x, t3, t3 + 3, t3 + 6, c);
-    if (d < best) {
-      best = d;
-      for (int t = 0; t < 3; ++t) {
-        bp[t] = ofp ? x[t] : c[t];
-        bq[t] = ofp ? c[t] : x[t];
-      }
-    }
-  }
-  for (int t = 0; t < 3; ++t) {
-    cp[t] = kx_add(bp[t], P[t]);
-    cq[t] = kx_add(bq[t], P[t]);
-  }
-  return best;
 }
 
 // lexicographic (d2, a, b) minimum across the warp; result in every lane

@@ -33,7 +33,7 @@
 #include <new>
 #include <vector>
 
-#include "kgpu_dist32.cuh"
+#include "kgpu_pairdist.cuh"
 
 namespace kgpu {
 kgpu_status record_error(kgpu_status code, const char* msg);
@@ -55,9 +55,8 @@ namespace kgpu {
 namespace {
 
 constexpr int kGW = 4;        // warps per block
-constexpr int kGStack = 512;  // node-pair stack entries per warp
-constexpr int kGJobs = 64;    // leaf-pair jobs
-constexpr int kGCand = 128;   // FP64 candidates (distance)
+constexpr int kGStack = kPStack;  // node-pair stack entries per warp
+constexpr int kGJobs = kPJobs;    // leaf-pair jobs
 
 struct GeomDev {
   const KNode* nodes;
@@ -90,19 +89,14 @@ struct __align__(16) GeomSmem {
   double T64[2][12];
   float T[2][12];
   float delta[2];
-  uint2 stack[kGStack];
-  uint32_t jobA[kGJobs], jobB[kGJobs], jobOff[kGJobs + 1];
-  uint32_t candA[kGCand], candB[kGCand];
-  float candD[kGCand];
-  uint8_t candS[kGCand];  // FP32-separated: the canonical overlap test is not needed
-  double pb2, pcp[3], pcq[3];
-  int pA, pB, phave;
+  PairSmem P;
 };
 
 // world placement of geometry triangle t (leaf order) in FP64
 __device__ __forceinline__ void tri_world64(const GeomDev& G, const double* T, int t, double* o)
 {
   const double* p = G.tri64 + 9 * (size_t)t;
+#pragma unroll 1
   for (int v = 0; v < 3; ++v) kx_xform_point(T, p + 3 * v, o + 3 * v);
 }
 
@@ -129,9 +123,6 @@ __device__ __forceinline__ float placement_err32(const float* T, float r)
   return kU * (6.f * nR * r + 5.f * nt) * 1.01f + 1e-30f;
 }
 
-// FP64 finalisation of distance candidates into the running lexicographic
-// best (pb2, pA, pB): pairs whose squared distance is below the bound, or
-// equal to the best with smaller (triangle of a, triangle of b)
 constexpr int kSeedMaxTris = 4096;  // geometries up to this size are scanned for a seed
 
 // An upper bound on the distance between the two placed surfaces: A's
@@ -170,86 +161,89 @@ __device__ __noinline__ float geom_seed(const GeomDev& GA, const GeomDev& GB, co
   return sqrtf(bo) * (1.f + 1e-5f) + 2.f * dd + 1e-6f;
 }
 
-__device__ __noinline__ void geom_flush(GeomSmem& S, const GeomDev& GA, const GeomDev& GB, int lane, int ncand,
-                                        float m32)
+// transforms of query b into S (both precisions) with their placement bounds;
+// false: a non-finite or huge entry (reported)
+__device__ __forceinline__ bool geom_load(GeomSmem& S, const GeomDev& GA, const GeomDev& GB, const GeomArgs& A, int b,
+                                          int lane)
 {
-  const float lim = m32 * (1.f + 2e-5f) + 1e-6f;
-  for (int base = 0; base < ncand; base += 32) {
-    const int k = base + lane;
-    double d2 = DBL_MAX;
-    int oa = INT_MAX, ob = INT_MAX;
-    double cp[3] = {0, 0, 0}, cq[3] = {0, 0, 0};
-    if (k < ncand && S.candD[k] <= lim) {
-      const int tA = (int)S.candA[k], tB = (int)S.candB[k];
-      double P[9], Q[9];
-      tri_world64(GA, S.T64[0], tA, P);
-      tri_world64(GB, S.T64[1], tB, Q);
-      float3 P32[3], Q32[3];
-      tri_world32(GA, S.T[0], tA, P32);
-      tri_world32(GB, S.T[1], tB, Q32);
-      const float thr2 = feature_thr2(P32, Q32, m32, S.delta[0] + S.delta[1]);
-      d2 = tri_dist2_masked64(P, Q, tri_feature_mask32(P32, Q32, thr2), S.candS[k] != 0, cp, cq);
-      oa = GA.tri_orig[tA];
-      ob = GB.tri_orig[tB];
-    }
-    int src;
-    double m2 = d2;
-    int ma = oa, mb = ob;
-    warp_lexmin(m2, ma, mb, src, lane);
-    const bool better = S.phave ? (m2 < S.pb2 || (m2 == S.pb2 && (ma < S.pA || (ma == S.pA && mb < S.pB))))
-                                : m2 < S.pb2;
-    __syncwarp();
-    if (m2 < DBL_MAX && better && lane == src) {
-      S.pb2 = d2;
-      S.pA = oa;
-      S.pB = ob;
-      S.phave = 1;
-      for (int c = 0; c < 3; ++c) { S.pcp[c] = cp[c]; S.pcq[c] = cq[c]; }
-    }
-    __syncwarp();
+  double tv = 0.0;
+  if (lane < 12) tv = A.Ta[(size_t)b * A.sa + lane];
+  else if (lane < 24) tv = A.Tb[(size_t)b * A.sb + lane - 12];
+  if (__any_sync(0xffffffffu, lane < 24 && !(fabs(tv) < 1e6))) {
+    if (lane == 0) set_status(A.status, KGPU_ERR_NOT_FINITE);
+    return false;
   }
+  if (lane < 12) { S.T64[0][lane] = tv; S.T[0][lane] = (float)tv; }
+  else if (lane < 24) { S.T64[1][lane - 12] = tv; S.T[1][lane - 12] = (float)tv; }
+  __syncwarp();
+  if (lane < 2) S.delta[lane] = placement_err32(S.T[lane], lane == 0 ? GA.r : GB.r);
+  __syncwarp();
+  return true;
 }
 
-template <bool DIST>
-__global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomDev GB, const GeomArgs A)
+__global__ void __launch_bounds__(kGW * 32) k_geom_distance(const GeomDev GA, const GeomDev GB, const GeomArgs A)
 {
   __shared__ GeomSmem smem[kGW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   GeomSmem& S = smem[warp];
-  const unsigned lt = lanemask_lt();
   const int nwarps = gridDim.x * kGW;
-  // collide: the FP32 threshold rounded up; distance: the FP32 search bound
-  const float m32 = A.m > 0.0 ? (float)A.m * 1.000001f + 1e-12f : 0.f;
+  const MeshView MA = {GA.nodes, GA.node_r, GA.tri32, GA.tri64, GA.tri_orig};
+  const MeshView MB = {GB.nodes, GB.node_r, GB.tri32, GB.tri64, GB.tri_orig};
   const float fcut = A.bound < 1e30 ? (float)A.bound * 1.000001f + 1e-7f : FLT_MAX;
+  PairCnt cnt;
 #pragma unroll 1
   for (int b = blockIdx.x * kGW + warp; b < A.B; b += nwarps) {
-    // ---- transforms
-    double tv = 0.0;
-    if (lane < 12) tv = A.Ta[(size_t)b * A.sa + lane];
-    else if (lane < 24) tv = A.Tb[(size_t)b * A.sb + lane - 12];
-    if (__any_sync(0xffffffffu, lane < 24 && !(fabs(tv) < 1e6))) {
-      if (lane == 0) set_status(A.status, KGPU_ERR_NOT_FINITE);
-      continue;
-    }
-    if (lane < 12) { S.T64[0][lane] = tv; S.T[0][lane] = (float)tv; }
-    else if (lane < 24) { S.T64[1][lane - 12] = tv; S.T[1][lane - 12] = (float)tv; }
-    __syncwarp();
-    if (lane < 2) S.delta[lane] = placement_err32(S.T[lane], lane == 0 ? GA.r : GB.r);
+    if (!geom_load(S, GA, GB, A, b, lane)) continue;
     if (lane == 0) {
-      S.stack[0] = make_uint2(0u, 0u);
       const double bb = kx_mul(A.bound, A.bound);
-      S.pb2 = bb > 1e-300 ? bb : 1e-300;
-      S.pA = S.pB = INT_MAX;
-      S.phave = 0;
+      S.P.b2 = bb > 1e-300 ? bb : 1e-300;
+      S.P.bA = S.P.bB = INT_MAX;
+      S.P.have = 0;
     }
     __syncwarp();
-    const float* TA = S.T[0];
-    const float* TB = S.T[1];
     const float dd = S.delta[0] + S.delta[1];
-    int top = (GA.ntri > 0 && GB.ntri > 0) ? 1 : 0, njobs = 0, ncand = 0;
+    // FP32 upper bound on the minimum (both geometries have triangles)
+    float run = fminf(fcut, geom_seed(GA, GB, S.T[0], S.T[1], lane, dd));
+    int certA = -1;
+    if (pair_distance<false, false>(S.P, MA, MB, 0, 0, S.T[0], S.T[1], S.T64[0], S.T64[1], dd, run, certA, lane, cnt,
+                                    [] {}) == 2 &&
+        lane == 0)
+      set_status(A.status, KGPU_ERR_OVERFLOW);
+    // ---- outputs
+    const bool found = S.P.have != 0;
+    const double dm = found ? kx_sqrt(S.P.b2) : 0.0;
+    if (lane == 0) {
+      A.d[b] = found ? kx_sub(dm, A.msum) : A.upper;
+      A.elem[2 * (size_t)b] = found ? S.P.bA : -1;
+      A.elem[2 * (size_t)b + 1] = found ? S.P.bB : -1;
+    }
+    if (lane < 6) A.cp[6 * (size_t)b + lane] = found ? (lane < 3 ? S.P.bcp[lane] : S.P.bcq[lane - 3]) : 0.0;
+    if (A.dir && lane < 3)
+      A.dir[3 * (size_t)b + lane] = found && dm > 0.0 ? kx_div(kx_sub(S.P.bcp[lane], S.P.bcq[lane]), dm) : 0.0;
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kGW * 32) k_geom_collide(const GeomDev GA, const GeomDev GB, const GeomArgs A)
+{
+  __shared__ GeomSmem smem[kGW];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  GeomSmem& G = smem[warp];
+  PairSmem& S = G.P;
+  const unsigned lt = lanemask_lt();
+  const int nwarps = gridDim.x * kGW;
+  // the FP32 threshold rounded up
+  const float m32 = A.m > 0.0 ? (float)A.m * 1.000001f + 1e-12f : 0.f;
+#pragma unroll 1
+  for (int b = blockIdx.x * kGW + warp; b < A.B; b += nwarps) {
+    if (!geom_load(G, GA, GB, A, b, lane)) continue;
+    if (lane == 0) S.stack[0] = make_uint2(0u, 0u);
+    __syncwarp();
+    const float* TA = G.T[0];
+    const float* TB = G.T[1];
+    const float dd = G.delta[0] + G.delta[1];
+    int top = (GA.ntri > 0 && GB.ntri > 0) ? 1 : 0, njobs = 0;
     bool hit = false;
-    float run = fcut;  // distance: FP32 upper bound on the minimum (warp-uniform)
-    if (DIST && top > 0) run = fminf(run, geom_seed(GA, GB, TA, TB, lane, dd));
 #pragma unroll 1
     while ((top > 0 || njobs > 0) && !hit) {
       if (njobs >= 16 || (top == 0 && njobs > 0)) {
@@ -273,8 +267,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
 #pragma unroll 1
         for (uint32_t base = 0; base < total && !hit; base += 32) {
           const uint32_t p = base + lane;
-          int tA = 0, tB = 0;
-          float3 P[3], Q[3];
+          bool h = false;
           if (p < total) {
             int lo = 0, hi = njobs - 1;
             while (lo < hi) {
@@ -283,64 +276,29 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
             }
             const uint32_t r = p - S.jobOff[lo];
             const uint32_t cb = (S.jobB[lo] >> 28) + 1;
-            tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
-            tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
+            const int tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
+            const int tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
+            float3 P[3], Q[3];
             tri_world32(GA, TA, tA, P);
             tri_world32(GB, TB, tB, Q);
-          }
-          if (!DIST) {
-            bool h = false;
-            if (p < total && !tri_separated32(P, Q, dd, m32)) {
+            if (!tri_separated32(P, Q, dd, m32)) {
               if (A.m == 0.0 && tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd)) {
                 h = true;
               } else {
                 // the band: the canonical FP64 decision
                 double P64[9], Q64[9];
-                tri_world64(GA, S.T64[0], tA, P64);
-                tri_world64(GB, S.T64[1], tB, Q64);
+                tri_world64(GA, G.T64[0], tA, P64);
+                tri_world64(GB, G.T64[1], tB, Q64);
                 if (A.m == 0.0) {
-                  h = kx_tri_tri_overlap(P64, Q64) != 0;
+                  h = tri_overlap64(P64, Q64) != 0;
                 } else {
                   double c1[3], c2[3];
-                  h = kx_tri_tri_dist2(P64, Q64, c1, c2) <= kx_mul(A.m, A.m);
+                  h = tri_dist2_masked64(P64, Q64, kFeatAll, false, c1, c2) <= kx_mul(A.m, A.m);
                 }
               }
             }
-            hit = __any_sync(0xffffffffu, h);
-          } else {
-            float d32 = FLT_MAX, e = 0.f;
-            if (p < total) {
-              float3 lo3 = P[0], hi3 = P[0];
-#pragma unroll
-              for (int k = 1; k < 6; ++k) {
-                const float3 v = k < 3 ? P[k] : Q[k - 3];
-                lo3 = make_float3(fminf(lo3.x, v.x), fminf(lo3.y, v.y), fminf(lo3.z, v.z));
-                hi3 = make_float3(fmaxf(hi3.x, v.x), fmaxf(hi3.y, v.y), fmaxf(hi3.z, v.z));
-              }
-              const float span = fmaxf(fmaxf(hi3.x - lo3.x, hi3.y - lo3.y), hi3.z - lo3.z);
-              e = dd + 128.f * kU * span + 1e-8f;
-              if (tri_axis_lb32(P, Q, span) - e > run * (1.f + 2e-5f) + 2.f * e) d32 = FLT_MAX;
-              else if (!tri_separated32(P, Q, dd, 0.f)) d32 = 0.f;
-              else d32 = sqrtf(tri_dist2_32(P, Q));
-            }
-            run = fminf(run, warp_min(d32 < FLT_MAX ? d32 + e : FLT_MAX));
-            const bool cand = d32 < FLT_MAX && d32 - e <= run * (1.f + 2e-5f);
-            const unsigned mc = __ballot_sync(0xffffffffu, cand);
-            if (ncand + __popc(mc) > kGCand) {
-              geom_flush(S, GA, GB, lane, ncand, run);
-              ncand = 0;
-              if (S.phave) run = fminf(run, (float)sqrt(S.pb2) * (1.f + 1e-6f));
-            }
-            if (cand) {
-              const int rr = ncand + __popc(mc & lt);
-              S.candA[rr] = (uint32_t)tA;
-              S.candB[rr] = (uint32_t)tB;
-              S.candD[rr] = d32 - e;
-              S.candS[rr] = d32 > 0.f;
-            }
-            ncand += __popc(mc);
-            __syncwarp();
           }
+          hit = __any_sync(0xffffffffu, h);
         }
         njobs = 0;
         continue;
@@ -364,17 +322,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
         const Box32 BB = xform_box(TB, nb.a, nb.b);
         const float slack = 4.f * kU * (fabsf(BA.c.x) + fabsf(BA.c.y) + fabsf(BA.c.z) + fabsf(BB.c.x) +
                                         fabsf(BB.c.y) + fabsf(BB.c.z) + 1.f);
-        bool keep;
-        if (!DIST) {
-          keep = boxes_overlap(BA, BB, dd + m32 + slack);
-        } else {
-          const float lb_box = box_dist32(BA, BB.c, BB.h) - dd * 1.7321f - slack;
-          const float cx = BA.c.x - BB.c.x, cy = BA.c.y - BB.c.y, cz = BA.c.z - BB.c.z;
-          const float lb_sph = sqrtf(cx * cx + cy * cy + cz * cz) * (1.f - 4.f * kU) -
-                               __ldg(GA.node_r + nodeA) - __ldg(GB.node_r + nodeB) - dd * 1.7321f - slack;
-          keep = fmaxf(lb_box, lb_sph) <= run * (1.f + 2e-5f) + 3.f * dd + 1e-5f;
-        }
-        if (keep) {
+        if (boxes_overlap(BA, BB, dd + m32 + slack)) {
           const int cntA = f2i(na.b.w), cntB = f2i(nb.b.w);
           const int ia = f2i(na.a.w), ib = f2i(nb.a.w);
           if (cntA > 0 && cntB > 0) {
@@ -396,9 +344,6 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
         // processed once 16 are pending (at most 16 + 32 < kGJobs); checked
         // so that an error is reported, not hidden
         if (lane == 0) set_status(A.status, KGPU_ERR_OVERFLOW);
-        top = 0;
-        njobs = 0;
-        ncand = 0;
         break;
       }
       if (outcome == 1) {
@@ -414,23 +359,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom(const GeomDev GA, const GeomD
       njobs += __popc(m2);
       __syncwarp();
     }
-    if (!DIST) {
-      if (lane == 0) A.hit[b] = hit ? 1 : 0;
-      continue;
-    }
-    if (ncand > 0) geom_flush(S, GA, GB, lane, ncand, run);
-    // ---- outputs
-    const bool found = S.phave != 0;
-    const double dm = found ? kx_sqrt(S.pb2) : 0.0;
-    if (lane == 0) {
-      A.d[b] = found ? kx_sub(dm, A.msum) : A.upper;
-      A.elem[2 * (size_t)b] = found ? S.pA : -1;
-      A.elem[2 * (size_t)b + 1] = found ? S.pB : -1;
-    }
-    if (lane < 6) A.cp[6 * (size_t)b + lane] = found ? (lane < 3 ? S.pcp[lane] : S.pcq[lane - 3]) : 0.0;
-    if (A.dir && lane < 3)
-      A.dir[3 * (size_t)b + lane] = found && dm > 0.0 ? kx_div(kx_sub(S.pcp[lane], S.pcq[lane]), dm) : 0.0;
-    __syncwarp();
+    if (lane == 0) A.hit[b] = hit ? 1 : 0;
   }
 }
 
@@ -611,7 +540,7 @@ extern "C" kgpu_status kgpu_geom_collide(kgpu_geom a, kgpu_geom b, const double*
   A.bound = 0.0;
   A.hit = hit;
   A.status = a->d_status;
-  k_geom<false><<<blocks_for(B), kGW * 32, 0, (cudaStream_t)stream>>>(dev_view(a), dev_view(b), A);
+  k_geom_collide<<<blocks_for(B), kGW * 32, 0, (cudaStream_t)stream>>>(dev_view(a), dev_view(b), A);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? KGPU_OK : record_error(KGPU_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -643,7 +572,7 @@ extern "C" kgpu_status kgpu_geom_distance(kgpu_geom a, kgpu_geom b, const double
   A.elem = elem;
   A.dir = dir;
   A.status = a->d_status;
-  k_geom<true><<<blocks_for(B), kGW * 32, 0, (cudaStream_t)stream>>>(dev_view(a), dev_view(b), A);
+  k_geom_distance<<<blocks_for(B), kGW * 32, 0, (cudaStream_t)stream>>>(dev_view(a), dev_view(b), A);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? KGPU_OK : record_error(KGPU_ERR_CUDA, cudaGetErrorString(e));
 }
