@@ -146,6 +146,49 @@ __device__ __noinline__ float pair_seed(DistSmem& S, const KWorldDev* __restrict
   return sqrtf(bo) * (1.f + 1e-5f) + 2.f * (S.delta[l] + W->eps_env + 2.f * W->eps_extra) + 1e-6f;
 }
 
+// FP32 bound of a vertex's depth inside object o against its exact value:
+// placement of the vertex, rounding of the planes and of their products
+__device__ __forceinline__ float depth_band(const KNode& ob, float dd)
+{
+  return dd + 32.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + fabsf(ob.b.x) + fabsf(ob.b.y) +
+                           fabsf(ob.b.z) + 1.f);
+}
+
+// Whether some vertex of link l may lie at least `need` >= 0 deep inside the
+// convex object o; otherwise the pair's signed distance is above -need (or
+// not negative, for need = 0).  One pass over the vertices, a few thousand
+// cycles; the pair's own evaluation (the search for a certified contact, then
+// its deepest vertex in FP64) takes a few hundred thousand.  Among boxes most
+// pairs a configuration still has to look at after its first contact are
+// shallower contacts: 32,768 terrain clearances 38.9 -> 27.4 ms with this test.
+__device__ __noinline__ bool may_be_deeper(const DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
+                                           int lane, int l, int o, float need)
+{
+  const KNode ob = W->enodes[W->obj_root[o]];
+  const float dd = S.delta[l] + W->eps_env + 2.f * W->eps_extra;
+  const float tolb = dd + 8.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + 1.f);
+  const float stop = need * (1.f - 1e-6f) - 2.f * depth_band(ob, dd);
+  const int ff = W->obj_leaf_first[o], fc = W->obj_leaf_count[o];
+  const int vf = R.link_vert_first[l], vc = R.link_vert_count[l];
+#pragma unroll 1
+  for (int base = 0; base < vc; base += 32) {
+    bool deep = false;
+    if (base + lane < vc) {
+      const float4 x = __ldg(W->lvert32 + vf + base + lane);
+      const float3 w = xform32(S.T[l], make_float3(x.x, x.y, x.z));
+      deep = fabsf(w.x - ob.a.x) <= ob.b.x + tolb && fabsf(w.y - ob.a.y) <= ob.b.y + tolb &&
+             fabsf(w.z - ob.a.z) <= ob.b.z + tolb;
+#pragma unroll 1
+      for (int f = ff; f < ff + fc && deep; ++f) {
+        const float4 pl = __ldg(W->eface32 + f);
+        deep = pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z) >= stop;
+      }
+    }
+    if (__any_sync(0xffffffffu, deep)) return true;
+  }
+  return false;
+}
+
 struct PairOut {
   int found;
   double d;
@@ -205,8 +248,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
     const KNode ob = W->enodes[W->obj_root[o]];
     const float tolb = dl + de + 8.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + 1.f);
     const int ff = W->obj_leaf_first[o], fc = W->obj_leaf_count[o];
-    const float ed = dl + de + 32.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + fabsf(ob.b.x) +
-                                           fabsf(ob.b.y) + fabsf(ob.b.z) + 1.f);
+    const float ed = depth_band(ob, dl + de);
     float lmax = -FLT_MAX;
     // pass 1: FP32 depths, lane-local maximum.  Each lane also keeps the (at
     // most two) vertices whose pass-1 value lies within 2 ed of its running
@@ -529,12 +571,19 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
           // not below minus the smallest half-extent of the object's box
           // (no point lies deeper inside a convex body that fits in the
           // box): once the best is at or under that, the pair can at most
-          // tie, which only a smaller (link, object) would win
-          const double dlow = W->obj_convex[o] ? -(double)fminf(fminf(W->enodes[W->obj_root[o]].b.x,
-                                                                       W->enodes[W->obj_root[o]].b.y),
-                                                                 W->enodes[W->obj_root[o]].b.z)
-                                               : 0.0;
-          if (bl >= 0 && (dlow > best || (dlow == best && !(l < bl || (l == bl && o < bo))))) continue;
+          // tie, which only a smaller (link, object) would win.  Nor can it
+          // go below minus the depth of the link's deepest vertex in it
+          if (bl >= 0) {
+            const bool convex = W->obj_convex[o] != 0, tie = l < bl || (l == bl && o < bo);
+            const double dlow = convex ? -(double)fminf(fminf(W->enodes[W->obj_root[o]].b.x,
+                                                              W->enodes[W->obj_root[o]].b.y),
+                                                        W->enodes[W->obj_root[o]].b.z)
+                                       : 0.0;
+            if (dlow > best || (dlow == best && !tie)) continue;
+            if (convex && best <= 0.0 && !(best == 0.0 && tie) &&
+                !may_be_deeper(S, W, R, lane, l, o, (float)-best))
+              continue;
+          }
           PairOut po;
           // the first pair has no running bound to prune with yet: seed it
           eval_pair(S, W, R, T64, fk64, lane, l, o, nextafter(best, 1e300), po, cnt,
