@@ -1095,14 +1095,15 @@ kgpu_status kgpu_softmin_grad(kgpu_world w, int32_t robot, const float* q, int32
   if (T < 0 || Wn < 1 || (T > 0 && (!q || !L))) return fail(KGPU_ERR_INVALID, "bad buffers");
   if (!(tau > 0)) return fail(KGPU_ERR_INVALID, "tau must be positive");
   if (!w->env) return fail(KGPU_ERR_EMPTY, "distance query without an environment (robotsim.cpp:1786-1787)");
-  size_t need = 2 * (size_t)T * Wn + T;
+  const int nl = w->robots[robot]->nlinks;
+  const size_t need = softmin_work_bytes(T, Wn, nl, w->env->nobj);
   if (need > w->scratch.dist_work_cap) {
     dfree(w->scratch.dist_work);
     w->scratch.dist_work_cap = 0;
-    CK(cudaMalloc((void**)&w->scratch.dist_work, need * sizeof(double)));
+    CK(cudaMalloc(&w->scratch.dist_work, need));
     w->scratch.dist_work_cap = need;
   }
-  return launch_status(launch_softmin(w->d_dev, w->scratch, robot, q, T, Wn, tau, L, dLdq, w->robots[robot]->nlinks,
+  return launch_status(launch_softmin(w->d_dev, w->scratch, robot, q, T, Wn, tau, L, dLdq, nl, w->env->nobj,
                                       w->scratch.dist_work, w->num_sms, (cudaStream_t)s),
                        "kgpu_softmin_grad");
 }

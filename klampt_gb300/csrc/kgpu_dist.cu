@@ -76,14 +76,34 @@ struct DistArgs {
   int* pair;           // [B*2]
   double* cp;          // [B*6]
   float* grad;         // [B*L] (mode 0: dd/dq, mode 2: unnormalised soft-min gradient)
-  const double* m_traj;  // mode 2: [T] trajectory minima
-  double* wsum;        // mode 2: [B] per-waypoint sums
+  // soft-min (modes 1 and 2): waypoints first .. first + B whose nseg is -1
+  // (their pairs did not fit the list), see SoftArgs
+  const int* nseg;
+  int first;
+  unsigned long long* mkey;  // [T] trajectory minima (double_key)
+  double* wsum;        // mode 2: [waypoints] sums
   int W;               // waypoints per trajectory
   double tau;
   unsigned int* head;
   uint2* scratch;
   int scratch_per_warp;
 };
+
+// doubles as unsigned integers in the same order, for atomicMin
+__device__ __forceinline__ unsigned long long double_key(double d)
+{
+  const unsigned long long u = (unsigned long long)__double_as_longlong(d);
+  return (u >> 63) ? ~u : u | (1ull << 63);
+}
+
+constexpr double kSoftCutoff = 1e3;  // pairs farther than this are not looked for
+
+// a trajectory's minimum from its key (all ones: none found yet)
+__device__ __forceinline__ double key_min(unsigned long long k)
+{
+  if (k == ~0ull) return kSoftCutoff;
+  return __longlong_as_double((long long)((k >> 63) ? k & ~(1ull << 63) : ~k));
+}
 
 struct DCnt {
   unsigned long long pairs = 0;
@@ -492,10 +512,29 @@ __device__ void pullback(DistSmem& S, const KRobotDev& R, int lane, float* g_out
   __syncwarp();
 }
 
-// MODE (A.mode): 0 minimum distance with closest points and gradient, 1
-// soft-min pass 1 (waypoint minima), 2 soft-min pass 2 (every pair below
-// m + K tau); one instantiation each, so that a launch carries only its
-// mode's code
+// adds a warp's counters to the world's: pairs are counted once per warp
+// (lane 0), the rest per lane
+__device__ __forceinline__ void count_pairs(const KWorldDev* __restrict__ W, const DCnt& cnt, int lane)
+{
+  unsigned long long nd = cnt.p.nodes, tp = cnt.p.tri, bd = cnt.p.fp64;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nd += __shfl_down_sync(0xffffffffu, nd, o);
+    tp += __shfl_down_sync(0xffffffffu, tp, o);
+    bd += __shfl_down_sync(0xffffffffu, bd, o);
+  }
+  if (lane == 0 && W->stats) {
+    atomicAdd(W->stats + 8, cnt.pairs);
+    atomicAdd(W->stats + 9, nd);
+    atomicAdd(W->stats + 10, tp);
+    atomicAdd(W->stats + 11, bd);
+  }
+}
+
+// MODE (A.mode): 0 minimum distance with closest points and gradient; 1 and
+// 2 the soft-min's two passes (trajectory minima, every pair below m + K tau)
+// for the waypoints whose pairs did not fit the soft-min's list; one
+// instantiation each, so that a launch carries only its mode's code
 template <int MODE>
 __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restrict__ W, const DistArgs A)
 {
@@ -514,7 +553,8 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     if (lane == 0) it = atomicAdd(A.head, 1u);
     it = __shfl_sync(0xffffffffu, it, 0);
     if (it >= (unsigned)A.B) break;
-    const int b = (int)it;
+    const int b = MODE == 0 ? (int)it : A.first + (int)it;
+    if (MODE != 0 && A.nseg[it] >= 0) continue;
     if (lane == 0) {
       S.item_qa = A.q + (size_t)b * nl;
       S.item_qb = nullptr;
@@ -624,15 +664,15 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
         lower = bound;
         round_bound = fmin(A.cutoff, round_bound * 4.0);
       }
-      if (lane == 0) {
+      if (MODE == 1) {
+        if (lane == 0 && bl >= 0) atomicMin(A.mkey + b / A.W, double_key(best));
+      } else if (lane == 0) {
         A.d[b] = bl >= 0 ? best : A.cutoff;
-        if (MODE == 0) {
-          A.pair[2 * b] = bl;
-          A.pair[2 * b + 1] = bo;
-          for (int i = 0; i < 3; ++i) {
-            A.cp[6 * b + i] = bl >= 0 ? bp.cp[i] : 0.0;
-            A.cp[6 * b + 3 + i] = bl >= 0 ? bp.cq[i] : 0.0;
-          }
+        A.pair[2 * b] = bl;
+        A.pair[2 * b + 1] = bo;
+        for (int i = 0; i < 3; ++i) {
+          A.cp[6 * b + i] = bl >= 0 ? bp.cp[i] : 0.0;
+          A.cp[6 * b + 3 + i] = bl >= 0 ? bp.cq[i] : 0.0;
         }
       }
       if (MODE == 0 && A.grad) {
@@ -642,7 +682,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     } else {
       // ---- soft-min pass 2: every pair below m + K tau
       const int t = b / A.W;
-      const double m = A.m_traj[t];
+      const double m = key_min(A.mkey[t]);
       const double bnd = m + kSoftK * A.tau;
       double sum = 0.0;
       const float fbnd = (float)fmax(bnd, 0.0) * 1.000001f + 1e-6f;
@@ -671,44 +711,360 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
       pullback(S, R, lane, A.grad ? A.grad + (size_t)b * nl : nullptr);
     }
   }
-  // counters: pairs are counted once per warp (lane 0), the rest per lane
-  unsigned long long nd = cnt.p.nodes, tp = cnt.p.tri, bd = cnt.p.fp64;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    nd += __shfl_down_sync(0xffffffffu, nd, o);
-    tp += __shfl_down_sync(0xffffffffu, tp, o);
-    bd += __shfl_down_sync(0xffffffffu, bd, o);
-  }
-  if (lane == 0 && W->stats) {
-    atomicAdd(W->stats + 8, cnt.pairs);
-    atomicAdd(W->stats + 9, nd);
-    atomicAdd(W->stats + 10, tp);
-    atomicAdd(W->stats + 11, bd);
-  }
+  count_pairs(W, cnt, lane);
 }
 
-// per-trajectory minimum of the waypoint minima
-__global__ void k_traj_min(const double* dwp, int T, int Wn, double* m)
+// ---- soft-min over a trajectory -----------------------------------------------
+// The pairs of all waypoints go into one list, and every warp of the GPU
+// takes pairs from it: one trajectory of 32 waypoints has a few thousand pairs
+// within 30 tau of its minimum, and one waypoint's are up to a few hundred, so
+// a warp per waypoint leaves the GPU idle or waiting for the last ones (one
+// trajectory 20-30 -> 1.7 ms, 200 trajectories 98.5 -> 54 ms).  Per chunk of
+// waypoints:
+//   k_soft_fk       FP32 and FP64 forward kinematics, kept for the chunk;
+//   k_soft_bound    an upper bound of each trajectory's minimum, from the
+//                   pairs nearest by their boxes at each waypoint;
+//   k_soft_gather   pairs within reach -> list (pass 1: of that bound, pass
+//                   2: of m + 30 tau);
+//   k_soft_eval     one pair per warp: pass 1 lowers the trajectory's exact
+//                   minimum, which prunes the pairs still to come; pass 2
+//                   stores distance, point and direction;
+//   k_soft_reduce   one warp per waypoint sums its pairs in the list order of
+//                   the waypoint (links, then objects as gathered), so results
+//                   do not depend on the scheduling.
+// A waypoint whose pairs do not fit (list or segment table full) is flagged
+// and done by one warp in k_dist<1> / k_dist<2>.
+constexpr int kSoftSegs = 128;        // list segments per waypoint (of up to kDPairs pairs)
+constexpr int kSoftChunk = 8192;      // waypoints per chunk
+constexpr int kSoftPerWaypoint = 256; // list capacity per waypoint of a chunk, on average
+
+struct SoftArgs {
+  int robot, nl;
+  const float* q;            // [waypoints, L]
+  int first, n;              // the chunk: waypoints first .. first + n
+  int W;                     // waypoints per trajectory
+  double tau;
+  // per waypoint of the chunk
+  float* T;                  // [n, nl, 12]
+  float* delta;              // [n, nl]
+  double* T64;               // [n, nl, 12]
+  int2* seg;                 // [n, kSoftSegs] (first pair, pairs)
+  int* nseg;                 // [n]; -1: did not fit
+  // per trajectory
+  unsigned int* ub;          // FP32 bits of an upper bound of the minimum's magnitude
+  unsigned long long* mkey;  // exact minimum (double_key)
+  // the list
+  uint2* item;               // (waypoint of the chunk or ~0, link << 27 | object)
+  float* lb;                 // box lower bound
+  double* d;                 // +inf: not below the bound
+  float4* p;                 // point on the link; .w unused
+  float4* u;                 // direction
+  int cap;
+  unsigned int* count;       // pairs in the list (may exceed cap)
+  unsigned int* head;        // work queue of k_soft_eval
+  double* wsum;              // [waypoints]
+  float* grad;               // [waypoints, L] or null
+};
+
+__global__ void __launch_bounds__(kDW * 32) k_soft_fk(const KWorldDev* __restrict__ W, const SoftArgs A)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T) return;
-  double v = dwp[(size_t)t * Wn];
-  for (int w = 1; w < Wn; ++w) v = fmin(v, dwp[(size_t)t * Wn + w]);
-  m[t] = v;
+  __shared__ double q64[kDW][kMaxLinks];
+  __shared__ double T64[kDW][kMaxLinks][12];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = blockIdx.x * kDW + warp;
+  if (w >= A.n) return;
+  const KRobotDev& R = W->robots[A.robot];
+  const int nl = A.nl;
+  const float q = lane < nl ? __ldg(A.q + (size_t)(A.first + w) * nl + lane) : 0.f;
+  const bool bad = __any_sync(0xffffffffu, lane < nl && !(fabsf(q) < 1.0e6f));
+  if (bad && lane == 0) set_status(W->status, KGPU_ERR_NOT_FINITE);
+  // (a bad waypoint goes on at q = 0: the query fails as a whole)
+  const float qv = bad ? 0.f : q;
+  float P[12], delta;
+  warp_fk32(R, lane, qv, 0.f, P, &delta);
+  if (lane < nl) {
+    const size_t at = (size_t)w * nl + lane;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) A.T[at * 12 + i] = P[i];
+    A.delta[at] = delta;
+    q64[warp][lane] = (double)qv;
+  }
+  __syncwarp();
+  warp_fk64(R, q64[warp], T64[warp], lane);
+  for (int i = lane; i < nl * 12; i += 32) A.T64[(size_t)w * nl * 12 + i] = T64[warp][i / 12][i % 12];
 }
 
-// L = m - tau log(sum), gradient normalised by the sum (waypoints in order)
-__global__ void k_softmin_final(const double* wsum, const double* m, int T, int Wn, int L, double tau,
+// the FP32 transforms of waypoint w of the chunk into S
+__device__ __forceinline__ void soft_load(DistSmem& S, const SoftArgs& A, int w, int lane)
+{
+  __syncwarp();
+  for (int i = lane; i < A.nl * 12; i += 32) S.T[i / 12][i % 12] = __ldg(A.T + (size_t)w * A.nl * 12 + i);
+  if (lane < A.nl) S.delta[lane] = __ldg(A.delta + (size_t)w * A.nl + lane);
+  __syncwarp();
+}
+
+// the trajectory's current upper bound: one read, broadcast (other warps lower
+// it meanwhile, and the lanes have to agree)
+__device__ __forceinline__ float soft_ub(const SoftArgs& A, int t, int lane)
+{
+  unsigned int u = 0;
+  if (lane == 0) u = *((volatile unsigned int*)(A.ub + t));
+  return __uint_as_float(__shfl_sync(0xffffffffu, u, 0));
+}
+
+__global__ void __launch_bounds__(kDW * 32, 2) k_soft_bound(const KWorldDev* __restrict__ W, const SoftArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  DistSmem& S = reinterpret_cast<DistSmem*>(smem_raw)[warp];
+  const KRobotDev& R = W->robots[A.robot];
+  DCnt cnt;
+#pragma unroll 1
+  for (int w = blockIdx.x * kDW + warp; w < A.n; w += gridDim.x * kDW) {
+    soft_load(S, A, w, lane);
+    const int t = (A.first + w) / A.W;
+    // pairs nearest by their boxes: the search radius grows until some are there
+    int np = 0;
+    float radius = 0.05f;
+#pragma unroll 1
+    while (np == 0) {
+      const float ub = soft_ub(A, t, lane);
+      const float reach = fminf(radius, ub);
+#pragma unroll 1
+      for (int l = 0; l < A.nl && np <= kDPairs - 32; ++l) {
+        if (R.link_root[l] < 0) continue;
+#pragma unroll 1
+        for (int g = 0; g < kMaxGroups && np <= kDPairs - 32; ++g) {
+          if (!((R.env_mask[l] >> g) & 1u) || W->group_root[g] < 0) continue;
+          int top = 1;
+          if (lane == 0) S.gstack[0] = (uint32_t)W->group_root[g];
+          __syncwarp();
+          np = gather_objects(S, W, R, lane, l, reach, -1.f, np, top);
+        }
+      }
+      if (radius >= (float)kSoftCutoff || radius >= ub) break;
+      radius *= 4.f;
+    }
+    // vertex-pair bounds of the three nearest; an object too large for one is
+    // evaluated (any distance found is an upper bound)
+#pragma unroll 1
+    for (int k = 0; k < min(np, 3); ++k) {
+      float v = FLT_MAX;
+      int idx = 0;
+      for (int i = lane; i < np; i += 32)
+        if (S.plb[i] < v) { v = S.plb[i]; idx = i; }
+      const float vm = warp_min(v);
+      const int at = __shfl_sync(0xffffffffu, idx, __ffs(__ballot_sync(0xffffffffu, v == vm)) - 1);
+      const int l = S.plink[at], o = S.pobj[at];
+      __syncwarp();
+      if (lane == 0) S.plb[at] = FLT_MAX;
+      __syncwarp();
+      const float ub = soft_ub(A, t, lane);
+      if (vm > ub) break;
+      float b = pair_seed(S, W, R, lane, l, o);
+      if (!(b < FLT_MAX)) {
+        PairOut po;
+        int fk64 = 1;
+        double(*T64)[12] = reinterpret_cast<double(*)[12]>(A.T64 + (size_t)w * A.nl * 12);
+        eval_pair(S, W, R, T64, fk64, lane, l, o, ub < 1e3f ? (double)ub : kSoftCutoff, po, cnt);
+        if (po.found) b = (float)fmax(po.d, 0.0) * 1.000001f + 1e-7f;
+      }
+      if (lane == 0 && b < ub) atomicMin(A.ub + t, __float_as_uint(b));
+    }
+  }
+}
+
+// PASS 1: pairs within the bound of the trajectory's minimum; 2: within m + 30 tau
+template <int PASS>
+__global__ void __launch_bounds__(kDW * 32) k_soft_gather(const KWorldDev* __restrict__ W, const SoftArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  DistSmem& S = reinterpret_cast<DistSmem*>(smem_raw)[warp];
+  const KRobotDev& R = W->robots[A.robot];
+#pragma unroll 1
+  for (int w = blockIdx.x * kDW + warp; w < A.n; w += gridDim.x * kDW) {
+    soft_load(S, A, w, lane);
+    const int t = (A.first + w) / A.W;
+    float reach;
+    if (PASS == 1) reach = fminf(__uint_as_float(A.ub[t]), (float)kSoftCutoff) * 1.00001f + 1e-6f;
+    else reach = (float)fmax(key_min(A.mkey[t]) + kSoftK * A.tau, 0.0) * 1.000001f + 1e-6f;
+    int ns = 0, np = 0;
+    bool fits = true;
+    auto put = [&] {
+      unsigned int base = 0;
+      if (lane == 0) base = atomicAdd(A.count, (unsigned)np);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      fits = fits && ns < kSoftSegs && base + (unsigned)np <= (unsigned)A.cap;
+      for (int k = lane; k < np; k += 32)
+        if (base + (unsigned)k < (unsigned)A.cap) {
+          A.item[base + k] = fits ? make_uint2((unsigned)w, ((unsigned)S.plink[k] << 27) | (unsigned)S.pobj[k])
+                                  : make_uint2(~0u, 0u);
+          A.lb[base + k] = S.plb[k];
+        }
+      if (fits && lane == 0) A.seg[(size_t)w * kSoftSegs + ns] = make_int2((int)base, np);
+      ++ns;
+      np = 0;
+      __syncwarp();
+    };
+#pragma unroll 1
+    for (int l = 0; l < A.nl && fits; ++l) {
+      if (R.link_root[l] < 0) continue;
+#pragma unroll 1
+      for (int g = 0; g < kMaxGroups && fits; ++g) {
+        if (!((R.env_mask[l] >> g) & 1u) || W->group_root[g] < 0) continue;
+        int top = 1;
+        if (lane == 0) S.gstack[0] = (uint32_t)W->group_root[g];
+        __syncwarp();
+        while (top > 0 && fits) {
+          np = gather_objects(S, W, R, lane, l, reach, -1.f, np, top);
+          if (top > 0) put();
+        }
+      }
+    }
+    if (np > 0 && fits) put();
+    if (lane == 0) A.nseg[w] = fits ? ns : -1;
+  }
+}
+
+template <int PASS>
+__global__ void __launch_bounds__(kDW * 32, 2) k_soft_eval(const KWorldDev* __restrict__ W, const SoftArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  DistSmem& S = reinterpret_cast<DistSmem*>(smem_raw)[warp];
+  const KRobotDev& R = W->robots[A.robot];
+  const unsigned total = min(*A.count, (unsigned)A.cap);
+  DCnt cnt;
+#pragma unroll 1
+  for (;;) {
+    unsigned int it = 0;
+    if (lane == 0) it = atomicAdd(A.head, 1u);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= total) break;
+    const uint2 e = A.item[it];
+    if (e.x == ~0u) continue;
+    const int w = (int)e.x, l = (int)(e.y >> 27), o = (int)(e.y & 0x7ffffffu);
+    const int t = (A.first + w) / A.W;
+    // (an increasing minimum is impossible: a stale value only prunes less)
+    unsigned long long key = 0;
+    if (lane == 0) key = PASS == 1 ? *((volatile unsigned long long*)(A.mkey + t)) : A.mkey[t];
+    const double m = key_min(__shfl_sync(0xffffffffu, key, 0));
+    __syncwarp();
+    if (lane < 12) S.T[l][lane] = __ldg(A.T + ((size_t)w * A.nl + l) * 12 + lane);
+    if (lane == 12) S.delta[l] = __ldg(A.delta + (size_t)w * A.nl + l);
+    __syncwarp();
+    double(*T64)[12] = reinterpret_cast<double(*)[12]>(A.T64 + (size_t)w * A.nl * 12);
+    int fk64 = 1;
+    PairOut po;
+    if (PASS == 1) {
+      if (A.lb[it] > (float)fmax(m, 0.0) * 1.00001f + 1e-6f) continue;
+      if (m <= 0.0 && (!W->obj_convex[o] || !may_be_deeper(S, W, R, lane, l, o, (float)-m))) continue;
+      const float ub = soft_ub(A, t, lane);
+      eval_pair(S, W, R, T64, fk64, lane, l, o, nextafter(m, 1e300), po, cnt, ub);
+      if (lane == 0 && po.found) {
+        atomicMin(A.mkey + t, double_key(po.d));
+        if (po.d < (double)ub) atomicMin(A.ub + t, __float_as_uint((float)fmax(po.d, 0.0) * 1.000001f + 1e-7f));
+      }
+    } else {
+      eval_pair(S, W, R, T64, fk64, lane, l, o, m + kSoftK * A.tau, po, cnt, pair_seed(S, W, R, lane, l, o));
+      if (lane == 0) {
+        A.d[it] = po.found ? po.d : DBL_MAX;
+        if (po.found) {
+          A.p[it] = make_float4((float)po.cp[0], (float)po.cp[1], (float)po.cp[2], 0.f);
+          A.u[it] = make_float4(po.dir[0], po.dir[1], po.dir[2], 0.f);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  count_pairs(W, cnt, lane);
+}
+
+// One warp per waypoint: e_k = exp(-(d_k - m) / tau) of its pairs in list
+// order, their sum and the weighted wrenches (lane l sums link l's), pulled
+// back through the chain.
+__global__ void __launch_bounds__(kDW * 32) k_soft_reduce(const KWorldDev* __restrict__ W, const SoftArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  DistSmem& S = reinterpret_cast<DistSmem*>(smem_raw)[warp];
+  const KRobotDev& R = W->robots[A.robot];
+  const int w = blockIdx.x * kDW + warp;
+  if (w >= A.n) return;
+  const int ns = A.nseg[w];
+  if (ns < 0) return;  // done by k_dist<2>
+  soft_load(S, A, w, lane);
+  const double m = key_min(A.mkey[(A.first + w) / A.W]);
+  double sum = 0.0;
+  float F[3] = {0.f, 0.f, 0.f}, M[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int s = 0; s < ns; ++s) {
+    const int2 sg = A.seg[(size_t)w * kSoftSegs + s];
+#pragma unroll 1
+    for (int base = 0; base < sg.y; base += 32) {
+      const int k = sg.x + base + lane;
+      const bool in = base + lane < sg.y;
+      const double d = in ? A.d[k] : DBL_MAX;
+      const bool found = d < DBL_MAX;
+      double e = 0.0;
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f), u = p;
+      int l = 0;
+      if (found) {
+        e = exp(-(d - m) / A.tau);
+        p = A.p[k];
+        u = A.u[k];
+        l = (int)(A.item[k].y >> 27);
+      }
+      unsigned todo = __ballot_sync(0xffffffffu, found);
+#pragma unroll 1
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const double es = __shfl_sync(0xffffffffu, e, src);
+        sum += es;
+        const float wgt = (float)es;
+        const float ux = wgt * __shfl_sync(0xffffffffu, u.x, src), uy = wgt * __shfl_sync(0xffffffffu, u.y, src),
+                    uz = wgt * __shfl_sync(0xffffffffu, u.z, src);
+        const float px = __shfl_sync(0xffffffffu, p.x, src), py = __shfl_sync(0xffffffffu, p.y, src),
+                    pz = __shfl_sync(0xffffffffu, p.z, src);
+        if (__shfl_sync(0xffffffffu, l, src) == lane) {
+          F[0] += ux; F[1] += uy; F[2] += uz;
+          M[0] += py * uz - pz * uy;
+          M[1] += pz * ux - px * uz;
+          M[2] += px * uy - py * ux;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    S.F[lane][c] = F[c];
+    S.M[lane][c] = M[c];
+  }
+  __syncwarp();
+  const size_t b = (size_t)A.first + w;
+  if (lane == 0) A.wsum[b] = sum;
+  pullback(S, R, lane, A.grad ? A.grad + b * A.nl : nullptr);
+}
+
+// L = m - tau log(sum) with the waypoints' sums in order, the gradient
+// normalised by the sum; one warp per trajectory
+__global__ void k_softmin_final(const double* wsum, const unsigned long long* mkey, int T, int Wn, int L, double tau,
                                 double* out, float* grad)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= T) return;
   double s = 0.0;
-  for (int w = 0; w < Wn; ++w) s += wsum[(size_t)t * Wn + w];
-  out[t] = m[t] - tau * log(s);
+#pragma unroll 1
+  for (int base = 0; base < Wn; base += 32) {
+    const double v = base + lane < Wn ? wsum[(size_t)t * Wn + base + lane] : 0.0;
+    for (int k = 0; k < min(32, Wn - base); ++k) s += __shfl_sync(0xffffffffu, v, k);
+  }
+  if (lane == 0) out[t] = key_min(mkey[t]) - tau * log(s);
   if (grad) {
     const float inv = (float)(1.0 / s);
-    for (int k = 0; k < Wn * L; ++k) grad[(size_t)t * Wn * L + k] *= inv;
+    for (size_t k = lane; k < (size_t)Wn * L; k += 32) grad[(size_t)t * Wn * L + k] *= inv;
   }
 }
 
@@ -961,13 +1317,14 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
 
 cudaError_t dist_init()
 {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_dist<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(DistSmem) * kDW));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_dist<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(DistSmem) * kDW));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_dist<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(DistSmem) * kDW));
-  if (e != cudaSuccess) return e;
+  const int smem = (int)(sizeof(DistSmem) * kDW);
+  const void* kernels[] = {(const void*)k_dist<0>,        (const void*)k_dist<1>,        (const void*)k_dist<2>,
+                           (const void*)k_soft_bound,     (const void*)k_soft_gather<1>, (const void*)k_soft_gather<2>,
+                           (const void*)k_soft_eval<1>,   (const void*)k_soft_eval<2>,   (const void*)k_soft_reduce};
+  for (const void* k : kernels) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
   return cudaFuncSetAttribute(k_self_dist, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(sizeof(SelfDistSmem) * kDW));
 }
@@ -995,39 +1352,123 @@ cudaError_t launch_distance(const KWorldDev* Wd, const Scratch& S, int robot, co
   return cudaGetLastError();
 }
 
+namespace {
+
+// device scratch of a soft-min call, carved out of one block
+struct SoftLayout {
+  int chunk, cap;  // waypoints per chunk, list capacity
+  size_t T, delta, T64, seg, nseg, ub, mkey, item, lb, d, p, u, wsum, count, bytes;
+};
+
+SoftLayout soft_layout(int T, int Wn, int nl, int nobj)
+{
+  SoftLayout L;
+  const size_t B = (size_t)T * Wn;
+  L.chunk = (int)(B < (size_t)kSoftChunk ? B : (size_t)kSoftChunk);
+  const size_t all = (size_t)L.chunk * nl * nobj, most = (size_t)L.chunk * kSoftPerWaypoint;
+  const size_t cap = all < most ? all : (most > 65536 ? most : (all < 65536 ? all : 65536));
+  L.cap = (int)cap;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + 255) / 256 * 256;
+    return here;
+  };
+  L.T = take(sizeof(float) * 12 * nl * L.chunk);
+  L.delta = take(sizeof(float) * nl * L.chunk);
+  L.T64 = take(sizeof(double) * 12 * nl * L.chunk);
+  L.seg = take(sizeof(int2) * kSoftSegs * L.chunk);
+  L.nseg = take(sizeof(int) * L.chunk);
+  L.item = take(sizeof(uint2) * cap);
+  L.lb = take(sizeof(float) * cap);
+  L.d = take(sizeof(double) * cap);
+  L.p = take(sizeof(float4) * cap);
+  L.u = take(sizeof(float4) * cap);
+  L.wsum = take(sizeof(double) * B);
+  L.ub = take(sizeof(unsigned int) * T);
+  L.mkey = take(sizeof(unsigned long long) * T);
+  L.count = take(4 * sizeof(unsigned int));
+  L.bytes = at;
+  return L;
+}
+
+}  // namespace
+
+size_t softmin_work_bytes(int T, int Wn, int nl, int nobj) { return soft_layout(T, Wn, nl, nobj).bytes; }
+
 cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int T, int Wn,
-                           double tau, double* L, float* dLdq, int nl, double* work, int num_sms, cudaStream_t s)
+                           double tau, double* L, float* dLdq, int nl, int nobj, void* work, int num_sms,
+                           cudaStream_t s)
 {
   if (T <= 0) return cudaSuccess;
+  const size_t smem = sizeof(DistSmem) * kDW;
   const int B = T * Wn;
-  double* dwp = work;            // [B]
-  double* mt = work + B;         // [T]
-  double* wsum = work + B + T;   // [B]
-  cudaError_t e = cudaMemsetAsync(S.counters + 8, 0, 2 * sizeof(unsigned int), s);
-  if (e != cudaSuccess) return e;
-  DistArgs A = {};
+  const SoftLayout lay = soft_layout(T, Wn, nl, nobj);
+  char* w = (char*)work;
+  SoftArgs A = {};
   A.robot = robot;
+  A.nl = nl;
   A.q = q;
-  A.B = B;
-  A.scratch = S.spill;
-  A.scratch_per_warp = (int)S.spill_per_warp;
-  // pass 1: waypoint minima (no cutoff)
-  A.mode = 1;
-  A.cutoff = 1e3;
-  A.d = dwp;
-  A.head = S.counters + 8;
-  k_dist<1><<<num_sms * 2, kDW * 32, sizeof(DistSmem) * kDW, s>>>(Wd, A);
-  k_traj_min<<<(T + 127) / 128, 128, 0, s>>>(dwp, T, Wn, mt);
-  // pass 2: every pair below m + K tau, unnormalised gradients
-  A.mode = 2;
-  A.m_traj = mt;
-  A.wsum = wsum;
   A.W = Wn;
   A.tau = tau;
+  A.T = (float*)(w + lay.T);
+  A.delta = (float*)(w + lay.delta);
+  A.T64 = (double*)(w + lay.T64);
+  A.seg = (int2*)(w + lay.seg);
+  A.nseg = (int*)(w + lay.nseg);
+  A.ub = (unsigned int*)(w + lay.ub);
+  A.mkey = (unsigned long long*)(w + lay.mkey);
+  A.item = (uint2*)(w + lay.item);
+  A.lb = (float*)(w + lay.lb);
+  A.d = (double*)(w + lay.d);
+  A.p = (float4*)(w + lay.p);
+  A.u = (float4*)(w + lay.u);
+  A.cap = lay.cap;
+  A.count = (unsigned int*)(w + lay.count);
+  A.head = A.count + 1;
+  A.wsum = (double*)(w + lay.wsum);
   A.grad = dLdq;
-  A.head = S.counters + 9;
-  k_dist<2><<<num_sms * 2, kDW * 32, sizeof(DistSmem) * kDW, s>>>(Wd, A);
-  k_softmin_final<<<(T + 127) / 128, 128, 0, s>>>(wsum, mt, T, Wn, nl, tau, L, dLdq);
+  // the flagged waypoints of a chunk, one warp each
+  DistArgs D = {};
+  D.robot = robot;
+  D.q = q;
+  D.cutoff = kSoftCutoff;
+  D.scratch = S.spill;
+  D.scratch_per_warp = (int)S.spill_per_warp;
+  D.nseg = A.nseg;
+  D.mkey = A.mkey;
+  D.wsum = A.wsum;
+  D.W = Wn;
+  D.tau = tau;
+  D.grad = dLdq;
+  D.head = A.count + 2;
+  // bounds start above every distance (0x7f7f7f7f is 3.4e38), minima as "none"
+  cudaError_t e = cudaMemsetAsync(A.ub, 0x7f, sizeof(unsigned int) * T, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(A.mkey, 0xff, sizeof(unsigned long long) * T, s);
+  for (int pass = 1; pass <= 2 && e == cudaSuccess; ++pass) {
+    for (int first = 0; first < B && e == cudaSuccess; first += lay.chunk) {
+      A.first = D.first = first;
+      A.n = D.B = B - first < lay.chunk ? B - first : lay.chunk;
+      const int warps = (A.n + kDW - 1) / kDW, some = warps < 2 * num_sms ? warps : 2 * num_sms;
+      if ((e = cudaMemsetAsync(A.count, 0, 4 * sizeof(unsigned int), s)) != cudaSuccess) return e;
+      // (one chunk: the transforms of pass 1 are still there in pass 2)
+      if (pass == 1 || lay.chunk < B) k_soft_fk<<<warps, kDW * 32, 0, s>>>(Wd, A);
+      if (pass == 1) {
+        k_soft_bound<<<some, kDW * 32, smem, s>>>(Wd, A);
+        k_soft_gather<1><<<some, kDW * 32, smem, s>>>(Wd, A);
+        k_soft_eval<1><<<2 * num_sms, kDW * 32, smem, s>>>(Wd, A);
+        k_dist<1><<<some, kDW * 32, smem, s>>>(Wd, D);
+      } else {
+        k_soft_gather<2><<<some, kDW * 32, smem, s>>>(Wd, A);
+        k_soft_eval<2><<<2 * num_sms, kDW * 32, smem, s>>>(Wd, A);
+        k_dist<2><<<some, kDW * 32, smem, s>>>(Wd, D);
+        k_soft_reduce<<<warps, kDW * 32, smem, s>>>(Wd, A);
+      }
+      e = cudaGetLastError();
+    }
+  }
+  if (e != cudaSuccess) return e;
+  k_softmin_final<<<(T + 3) / 4, 128, 0, s>>>(A.wsum, A.mkey, T, Wn, nl, tau, L, dLdq);
   return cudaGetLastError();
 }
 

@@ -145,8 +145,8 @@ struct Scratch {
   int* edge_perm = nullptr;
   int* edge_meta = nullptr;          // 4 meta words, fill counters, count_ge (2 x (kMaxSteps+2))
   size_t edge_cap = 0;
-  double* dist_work = nullptr;       // soft-min per-waypoint minima, sums, trajectory minima
-  size_t dist_work_cap = 0;
+  void* dist_work = nullptr;         // soft-min pair list, transforms of a chunk, sums, minima
+  size_t dist_work_cap = 0;          // bytes
   // launch setting carried with the scratch: environment nodes a staged
   // engine block copies to shared memory (0: the unstaged kernels)
   int stage_nodes = 0;
@@ -324,8 +324,9 @@ cudaError_t launch_distance(const KWorldDev* Wd, const Scratch& S, int robot, co
 cudaError_t launch_self_distance(const KWorldDev* Wd, int robot, const float* q, int B, double cutoff, double* d,
                                  int* pair, double* cp, float* grad, double* dpair, int all_pairs, int num_sms,
                                  cudaStream_t s);
-// work: 2*T*Wn + T doubles of device scratch
+// work: softmin_work_bytes() of device scratch
+size_t softmin_work_bytes(int T, int Wn, int nl, int nobj);
 cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int T,
-                           int Wn, double tau, double* L, float* dLdq, int nl, double* work,
+                           int Wn, double tau, double* L, float* dLdq, int nl, int nobj, void* work,
                            int num_sms, cudaStream_t s);
 }  // namespace kgpu
