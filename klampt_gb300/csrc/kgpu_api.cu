@@ -1120,7 +1120,7 @@ kgpu_status kgpu_ik_solve(kgpu_world w, int32_t robot, int32_t B, float* q, cons
   if (!links && (link < 0 || link >= nl)) return fail(KGPU_ERR_INVALID, "link %d out of range [0,%d)", link, nl);
   if (max_iters < 0 || !(tol > 0)) return fail(KGPU_ERR_INVALID, "max_iters must be >= 0 and tol > 0");
   return launch_status(launch_ik(w->d_dev, robot, B, q, links, link, plocal, ptarget, Rtarget, max_iters, tol, ok,
-                                 residual, iters, (cudaStream_t)s),
+                                 residual, iters, nl, w->num_sms, (cudaStream_t)s),
                        "kgpu_ik_solve");
 }
 

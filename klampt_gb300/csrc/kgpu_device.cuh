@@ -156,6 +156,8 @@ __device__ __forceinline__ void joint_local32(const KRobotDev& R, int i, float q
 // warp_fk32_group runs G = 32 / L independent configurations at once: lanes
 // [g L, g L + L) hold configuration g, lane g L + i link i (active when
 // `valid`); warp_fk32 is the single-configuration case (L = 32).
+// ERR = false: transforms only (delta is not written).
+template <bool ERR = true>
 __device__ __forceinline__ void warp_fk32_group(const KRobotDev& R, int lane, int L, bool valid, float q,
                                                 float e_q, float* P, float* delta)
 {
@@ -175,20 +177,26 @@ __device__ __forceinline__ void warp_fk32_group(const KRobotDev& R, int lane, in
 #pragma unroll
     for (int k = 0; k < 12; ++k) Pa[k] = __shfl_sync(0xffffffffu, P[k], src);
     const int anc2 = __shfl_sync(0xffffffffu, anc, src);
-    const float ra = __shfl_sync(0xffffffffu, rho, src);
-    const float ta = __shfl_sync(0xffffffffu, tau, src);
+    float ra = 0.f, ta = 0.f;
+    if (ERR) {
+      ra = __shfl_sync(0xffffffffu, rho, src);
+      ta = __shfl_sync(0xffffffffu, tau, src);
+    }
     if (anc >= 0) {
       float o[12];
       compose32(Pa, P, o);
-      float r2, t2;
-      compose_err(ra, ta, tnorm(Pa), rho, tau, tnorm(P), &r2, &t2);
-      rho = r2;
-      tau = t2;
+      if (ERR) {
+        float r2, t2;
+        compose_err(ra, ta, tnorm(Pa), rho, tau, tnorm(P), &r2, &t2);
+        rho = r2;
+        tau = t2;
+      }
 #pragma unroll
       for (int k = 0; k < 12; ++k) P[k] = o[k];
       anc = anc2;
     }
   }
+  if (!ERR) return;
   const float rl = valid ? R.link_r[link] : 0.f;
   *delta = (rho * rl + tau + kU * (12.f * rl + 6.f * tnorm(P))) * 1.001f + 1e-9f;
 }

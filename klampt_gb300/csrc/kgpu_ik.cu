@@ -1,4 +1,5 @@
-// kgpu_ik.cu — batched inverse kinematics, one warp per problem.
+// kgpu_ik.cu — batched inverse kinematics, 32 / L problems per warp (L: the
+// robot's links rounded up to 8, 16 or 32).
 //
 // Replaces IKSolver.solve over IKObjective point / transform constraints
 // (Python/klampt/src/robotik.cpp:556-689; KrisLibrary RobotIKSolver, absent
@@ -35,27 +36,32 @@ struct IkArgs {
   uint8_t* ok;           // [B]
   float* residual;       // [B] max |e_i| at the result
   int* iters;            // [B] iterations used (may be null)
+  int per_block;         // problems of a block
 };
 
-__device__ __forceinline__ float warp_sum(float v)
+// sum over a group of L lanes, the first lane's value for all (the lanes'
+// orders differ)
+template <int L>
+__device__ __forceinline__ float group_sum(float v, int gbase)
 {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return __shfl_sync(0xffffffffu, v, gbase);
 }
 
-// residual of link li at the FP32 transforms held in lanes (P of lane li)
-__device__ __forceinline__ void ik_residual(const float* P, int li, float3 pl, const float* pt, const float* Rt,
-                                            int m, float* e)
+// residual of the link in lane `src` at the FP32 transforms held in lanes
+template <int M>
+__device__ __forceinline__ void ik_residual(const float* P, int src, float3 pl, const float* pt, const float* Rt,
+                                            float* e)
 {
   float T[12];
 #pragma unroll
-  for (int k = 0; k < 12; ++k) T[k] = __shfl_sync(0xffffffffu, P[k], li);
+  for (int k = 0; k < 12; ++k) T[k] = __shfl_sync(0xffffffffu, P[k], src);
   const float3 p = xform32(T, pl);
   e[0] = p.x - pt[0];
   e[1] = p.y - pt[1];
   e[2] = p.z - pt[2];
-  if (m == 6) {
+  if (M == 6) {
     // 1/2 sum over columns k of R*_k x R_k
     float ex = 0.f, ey = 0.f, ez = 0.f;
 #pragma unroll
@@ -66,66 +72,107 @@ __device__ __forceinline__ void ik_residual(const float* P, int li, float3 pl, c
       ey += az * bx - ax * bz;
       ez += ax * by - ay * bx;
     }
-    e[3] = 0.5f * ex;
-    e[4] = 0.5f * ey;
-    e[5] = 0.5f * ez;
+    e[M - 3] = 0.5f * ex;
+    e[M - 2] = 0.5f * ey;
+    e[M - 1] = 0.5f * ez;
   }
 }
 
-__global__ void __launch_bounds__(256) k_ik(const KWorldDev* __restrict__ W, const IkArgs A)
+// M: residual entries (3 position, 6 position and rotation).  A group of L
+// lanes (lane g L + i: link i) iterates on its problem and takes the block's
+// next one when it is done, so that the few problems that run to the iteration
+// limit do not hold up the others of their warp.  Bound by instruction issue
+// and the dependent shuffle and division chains of an iteration (M and L as
+// parameters let the 21 group sums overlap: 890 -> 750 us).  One warp per
+// problem left 25 of 32 lanes idle for a 7-link arm: 65,536 point + rotation
+// problems 1,660 -> 750 us for the call, 640 us of it the kernel, whose last
+// part is the 1% of the problems that run to 100 iterations (putting those
+// off until the others are done changed nothing).
+template <int M, int L>
+__global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, const IkArgs A)
 {
   const int lane = threadIdx.x & 31;
-  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (b >= A.B) return;
   const KRobotDev& R = W->robots[A.robot];
   const int nl = R.nlinks;
-  const int li = A.links ? __ldg(A.links + b) : A.link_all;
-  if (li < 0 || li >= nl) {
-    if (lane == 0) set_status(W->status, KGPU_ERR_INVALID);
-    return;
-  }
-  const int m = A.Rtarget ? 6 : 3;
-  const float3 pl = make_float3(A.plocal[3 * (size_t)b], A.plocal[3 * (size_t)b + 1], A.plocal[3 * (size_t)b + 2]);
-  float pt[3], Rt[9];
-  for (int k = 0; k < 3; ++k) pt[k] = A.ptarget[3 * (size_t)b + k];
-  for (int k = 0; k < 9; ++k) Rt[k] = A.Rtarget ? A.Rtarget[9 * (size_t)b + k] : 0.f;
-  // active DOFs: the link and its ancestors (other columns of J are 0)
-  bool active = false;
-  if (lane < nl)
-    for (int j = li; j >= 0; j = R.parents[j])
-      if (j == lane) { active = true; break; }
-  active = active && R.jtype[lane < nl ? lane : 0] != KX_JOINT_WELD;
-  const float lo = lane < nl ? R.qmin[lane] : 0.f, hi = lane < nl ? R.qmax[lane] : 0.f;
-  float q = lane < nl ? A.q[(size_t)b * nl + lane] : 0.f;
-  q = fminf(fmaxf(q, lo), hi);
+  const int link = lane & (L - 1), gbase = lane & ~(L - 1);
+  const bool valid = link < nl;
+  const int first = blockIdx.x * A.per_block, count = min(A.per_block, A.B - first);
+  __shared__ int taken;
+  if (threadIdx.x == 0) taken = 0;
+  __syncthreads();
+  const float lo = valid ? R.qmin[link] : 0.f, hi = valid ? R.qmax[link] : 0.f;
+  const bool weld = !valid || R.jtype[link] == KX_JOINT_WELD;
+  const bool revolute = valid && R.jtype[link] == KX_JOINT_REVOLUTE;
 
-  float P[12], delta, e[6];
-  warp_fk32(R, lane, q, 0.f, P, &delta);
-  ik_residual(P, li, pl, pt, Rt, m, e);
-  float E = 0.f, emax = 0.f;
-  for (int a = 0; a < m; ++a) {
-    E += e[a] * e[a];
-    emax = fmaxf(emax, fabsf(e[a]));
-  }
-  float mu = 1e-4f;
-  int it = 0;
+  int b = -1, it = 0, li = 0;   // b: problem, -1: none
+  bool more = true, start = false, active = false;
+  float3 pl = make_float3(0.f, 0.f, 0.f);
+  float pt[3] = {0.f, 0.f, 0.f}, Rt[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) Rt[k] = 0.f;
+  float q = 0.f, P[12], e[M], E = 0.f, emax = 0.f, mu = 0.f;
+#pragma unroll
+  for (int k = 0; k < 12; ++k) P[k] = 0.f;
+#pragma unroll
+  for (int a = 0; a < M; ++a) e[a] = 0.f;
 #pragma unroll 1
-  for (; it < A.max_iters && emax > A.tol; ++it) {
-    // column `lane` of J at q (angular rows 0-2, linear rows 3-5 as in
+  for (;;) {
+    // ---- the block's next problem for groups without one
+    if (__any_sync(0xffffffffu, b < 0 && more)) {
+      int nb = -1;
+      if (b < 0 && more && link == 0) nb = atomicAdd(&taken, 1);
+      nb = __shfl_sync(0xffffffffu, nb, gbase);
+      if (b < 0 && more) {
+        if (nb >= count) {
+          more = false;
+        } else {
+          nb += first;
+          li = A.links ? __ldg(A.links + nb) : A.link_all;
+          if (li < 0 || li >= nl) {
+            if (link == 0) set_status(W->status, KGPU_ERR_INVALID);
+            li = 0;
+          } else {
+            b = nb;
+            start = true;
+            it = 0;
+            mu = 1e-4f;
+            pl = make_float3(A.plocal[3 * (size_t)b], A.plocal[3 * (size_t)b + 1], A.plocal[3 * (size_t)b + 2]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) pt[k] = A.ptarget[3 * (size_t)b + k];
+            if (M == 6) {
+#pragma unroll
+              for (int k = 0; k < 9; ++k) Rt[k] = A.Rtarget[9 * (size_t)b + k];
+            }
+            // active DOFs: the link and its ancestors (other columns of J are 0)
+            active = false;
+            if (!weld)
+              for (int j = li; j >= 0; j = R.parents[j])
+                if (j == link) { active = true; break; }
+            q = valid ? A.q[(size_t)b * nl + link] : 0.f;
+            q = fminf(fmaxf(q, lo), hi);
+          }
+        }
+      }
+    }
+    if (!__any_sync(0xffffffffu, b >= 0)) {
+      if (!__any_sync(0xffffffffu, more)) break;
+      continue;
+    }
+    // ---- column `link` of J at q (angular rows 0-2, linear rows 3-5 as in
     // k_jacobian); the residual orders position first, so row a of the
     // system is linear row a (a < 3) and angular row a - 3 (a >= 3)
     float c[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     {
       float Ti[12];
 #pragma unroll
-      for (int k = 0; k < 12; ++k) Ti[k] = __shfl_sync(0xffffffffu, P[k], li);
+      for (int k = 0; k < 12; ++k) Ti[k] = __shfl_sync(0xffffffffu, P[k], gbase + li);
       const float3 p = xform32(Ti, pl);
       if (active) {
-        const float ax = R.axis[lane][0], ay = R.axis[lane][1], az = R.axis[lane][2];
+        const float ax = R.axis[link][0], ay = R.axis[link][1], az = R.axis[link][2];
         const float wx = P[0] * ax + P[1] * ay + P[2] * az;
         const float wy = P[3] * ax + P[4] * ay + P[5] * az;
         const float wz = P[6] * ax + P[7] * ay + P[8] * az;
-        if (R.jtype[lane] == KX_JOINT_REVOLUTE) {
+        if (revolute) {
           const float rx = p.x - P[9], ry = p.y - P[10], rz = p.z - P[11];
           c[0] = wy * rz - wz * ry;
           c[1] = wz * rx - wx * rz;
@@ -136,76 +183,90 @@ __global__ void __launch_bounds__(256) k_ik(const KWorldDev* __restrict__ W, con
         }
       }
     }
-    // A = J J^T + mu I (symmetric, lower triangle), y = A^-1 e by Cholesky,
-    // every lane the same values
-    float Am[21];
-    int k = 0;
-    for (int r = 0; r < m; ++r)
-      for (int s = 0; s <= r; ++s)  // lane 0's sum for all: the lanes' orders differ
-        Am[k++] = __shfl_sync(0xffffffffu, warp_sum(c[r] * c[s]), 0) + (r == s ? mu : 0.f);
-    float y[6];
+    // A = J J^T + mu I (symmetric, lower triangle), y = A^-1 e by Cholesky in
+    // place, every lane of the group the same values
+    float Lc[M * (M + 1) / 2];
+#pragma unroll
+    for (int r = 0; r < M; ++r)
+#pragma unroll
+      for (int s = 0; s <= r; ++s)
+        Lc[r * (r + 1) / 2 + s] = group_sum<L>(c[r] * c[s], gbase) + (r == s ? mu : 0.f);
+    float y[M];
     bool spd = true;
-    {
-      float Lc[21];
-      k = 0;
-      for (int r = 0; r < m; ++r) {
-        for (int s = 0; s <= r; ++s, ++k) {
-          float v = Am[k];
-          for (int t = 0; t < s; ++t) v -= Lc[r * (r + 1) / 2 + t] * Lc[s * (s + 1) / 2 + t];
-          if (s == r) {
-            spd = spd && v > 0.f;
-            Lc[k] = sqrtf(fmaxf(v, 1e-30f));
-          } else {
-            Lc[k] = v / Lc[s * (s + 1) / 2 + s];
-          }
+#pragma unroll
+    for (int r = 0; r < M; ++r)
+#pragma unroll
+      for (int s = 0; s <= r; ++s) {
+        float v = Lc[r * (r + 1) / 2 + s];
+#pragma unroll
+        for (int t = 0; t < s; ++t) v -= Lc[r * (r + 1) / 2 + t] * Lc[s * (s + 1) / 2 + t];
+        if (s == r) {
+          spd = spd && v > 0.f;
+          Lc[r * (r + 1) / 2 + s] = sqrtf(fmaxf(v, 1e-30f));
+        } else {
+          Lc[r * (r + 1) / 2 + s] = v / Lc[s * (s + 1) / 2 + s];
         }
       }
-      float z[6];
-      for (int r = 0; r < m; ++r) {
+    {
+      float z[M];
+#pragma unroll
+      for (int r = 0; r < M; ++r) {
         float v = e[r];
+#pragma unroll
         for (int t = 0; t < r; ++t) v -= Lc[r * (r + 1) / 2 + t] * z[t];
         z[r] = v / Lc[r * (r + 1) / 2 + r];
       }
-      for (int r = m - 1; r >= 0; --r) {
+#pragma unroll
+      for (int r = M - 1; r >= 0; --r) {
         float v = z[r];
-        for (int t = r + 1; t < m; ++t) v -= Lc[t * (t + 1) / 2 + r] * y[t];
+#pragma unroll
+        for (int t = r + 1; t < M; ++t) v -= Lc[t * (t + 1) / 2 + r] * y[t];
         y[r] = v / Lc[r * (r + 1) / 2 + r];
       }
     }
-    if (!spd) {
-      mu *= 8.f;
-      if (mu > 1e6f) break;
-      continue;
-    }
     float dq = 0.f;
-    for (int r = 0; r < m; ++r) dq -= c[r] * y[r];
-    const float qn = lane < nl ? fminf(fmaxf(q + dq, lo), hi) : 0.f;
-    float Pn[12], dn, en[6];
-    warp_fk32(R, lane, qn, 0.f, Pn, &dn);
-    ik_residual(Pn, li, pl, pt, Rt, m, en);
+#pragma unroll
+    for (int r = 0; r < M; ++r) dq -= c[r] * y[r];
+    // ---- the trial step (a new problem: its start; not positive definite: none)
+    const float qn = !valid ? 0.f : (start || !spd ? q : fminf(fmaxf(q + dq, lo), hi));
+    float Pn[12], en[M];
+    warp_fk32_group<false>(R, lane, L, valid, qn, 0.f, Pn, nullptr);
+    ik_residual<M>(Pn, gbase + li, pl, pt, Rt, en);
     float En = 0.f, enmax = 0.f;
-    for (int a = 0; a < m; ++a) {
+#pragma unroll
+    for (int a = 0; a < M; ++a) {
       En += en[a] * en[a];
       enmax = fmaxf(enmax, fabsf(en[a]));
     }
-    if (En < E) {
+    bool done = false;
+    if (start || (spd && En < E)) {
       q = qn;
 #pragma unroll
       for (int t = 0; t < 12; ++t) P[t] = Pn[t];
-      for (int a = 0; a < m; ++a) e[a] = en[a];
+#pragma unroll
+      for (int a = 0; a < M; ++a) e[a] = en[a];
       E = En;
       emax = enmax;
-      mu = fmaxf(mu * 0.25f, 1e-10f);
+      if (!start) {
+        mu = fmaxf(mu * 0.25f, 1e-10f);
+        ++it;
+      }
     } else {
       mu *= 8.f;
-      if (mu > 1e6f) break;
+      if (mu > 1e6f) done = true;  // gives up
+      else ++it;
     }
-  }
-  if (lane < nl) A.q[(size_t)b * nl + lane] = q;
-  if (lane == 0) {
-    A.ok[b] = emax <= A.tol ? 1 : 0;
-    A.residual[b] = emax;
-    if (A.iters) A.iters[b] = it;
+    start = false;
+    done = done || !(it < A.max_iters && emax > A.tol);
+    if (b >= 0 && done) {
+      if (valid) A.q[(size_t)b * nl + link] = q;
+      if (link == 0) {
+        A.ok[b] = emax <= A.tol ? 1 : 0;
+        A.residual[b] = emax;
+        if (A.iters) A.iters[b] = it;
+      }
+      b = -1;
+    }
   }
 }
 
@@ -213,7 +274,8 @@ __global__ void __launch_bounds__(256) k_ik(const KWorldDev* __restrict__ W, con
 
 cudaError_t launch_ik(const KWorldDev* W, int robot, int B, float* q, const int* links, int link_all,
                       const float* plocal, const float* ptarget, const float* Rtarget, int max_iters, float tol,
-                      uint8_t* ok, float* residual, int* iters, cudaStream_t s)
+                      uint8_t* ok, float* residual, int* iters, int nlinks, int num_sms,
+                      cudaStream_t s)
 {
   if (B <= 0) return cudaSuccess;
   IkArgs A;
@@ -230,8 +292,23 @@ cudaError_t launch_ik(const KWorldDev* W, int robot, int B, float* q, const int*
   A.ok = ok;
   A.residual = residual;
   A.iters = iters;
-  const int threads = 256;
-  k_ik<<<(int)(((long long)B * 32 + threads - 1) / threads), threads, 0, s>>>(W, A);
+  // one wave of blocks (2 of 8 warps per SM), each with its share of the
+  // problems: the queue is the block's own, so calls on several streams do not
+  // share anything.  Fewer problems than groups: one each
+  const int threads = 256, groups = threads / 32 * (nlinks <= 8 ? 4 : (nlinks <= 16 ? 2 : 1));
+  const int share = (B + 2 * num_sms - 1) / (2 * num_sms);
+  A.per_block = share > groups ? share : groups;
+  const int blocks = (B + A.per_block - 1) / A.per_block;
+  if (nlinks <= 8) {
+    if (Rtarget) k_ik<6, 8><<<blocks, threads, 0, s>>>(W, A);
+    else k_ik<3, 8><<<blocks, threads, 0, s>>>(W, A);
+  } else if (nlinks <= 16) {
+    if (Rtarget) k_ik<6, 16><<<blocks, threads, 0, s>>>(W, A);
+    else k_ik<3, 16><<<blocks, threads, 0, s>>>(W, A);
+  } else {
+    if (Rtarget) k_ik<6, 32><<<blocks, threads, 0, s>>>(W, A);
+    else k_ik<3, 32><<<blocks, threads, 0, s>>>(W, A);
+  }
   return cudaGetLastError();
 }
 
