@@ -81,13 +81,11 @@ __device__ __forceinline__ void ik_residual(const float* P, int src, float3 pl, 
 // M: residual entries (3 position, 6 position and rotation).  A group of L
 // lanes (lane g L + i: link i) iterates on its problem and takes the block's
 // next one when it is done, so that the few problems that run to the iteration
-// limit do not hold up the others of their warp.  Bound by instruction issue
-// and the dependent shuffle and division chains of an iteration (M and L as
-// parameters let the 21 group sums overlap: 890 -> 750 us).  One warp per
-// problem left 25 of 32 lanes idle for a 7-link arm: 65,536 point + rotation
-// problems 1,660 -> 750 us for the call, 640 us of it the kernel, whose last
-// part is the 1% of the problems that run to 100 iterations (putting those
-// off until the others are done changed nothing).
+// limit do not hold up the others of their warp.  Bound by the dependent
+// shuffle, division and square root chains of an iteration (M and L as
+// parameters let the 21 group sums overlap).  One warp per problem left 25 of
+// 32 lanes idle for a 7-link arm: 65,536 point + rotation problems 1,650 ->
+// 532 us for the call, 9,000 552 -> 377 us.
 template <int M, int L>
 __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, const IkArgs A)
 {
@@ -110,11 +108,11 @@ __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, 
   float pt[3] = {0.f, 0.f, 0.f}, Rt[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) Rt[k] = 0.f;
-  float q = 0.f, P[12], e[M], E = 0.f, emax = 0.f, mu = 0.f;
+  float q = 0.f, P[12], e[M], E = 0.f, emax = 0.f, mu = 1.f;
 #pragma unroll
   for (int k = 0; k < 12; ++k) P[k] = 0.f;
 #pragma unroll
-  for (int a = 0; a < M; ++a) e[a] = 0.f;
+  for (int a = 0; a < M; ++a) e[a] = 0.1f;
 #pragma unroll 1
   for (;;) {
     // ---- the block's next problem for groups without one
@@ -167,7 +165,13 @@ __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, 
 #pragma unroll
       for (int k = 0; k < 12; ++k) Ti[k] = __shfl_sync(0xffffffffu, P[k], gbase + li);
       const float3 p = xform32(Ti, pl);
-      if (active) {
+      if (b < 0) {
+        // a group without a problem computes along: on harmless values, for
+        // zeros, infinities or NaN would take the divisions' slow paths, which
+        // the whole warp waits for (2x the time of an iteration)
+#pragma unroll
+        for (int r = 0; r < 6; ++r) c[r] = 0.1f + 0.02f * (float)((link + 3 * r) & 7);
+      } else if (active) {
         const float ax = R.axis[link][0], ay = R.axis[link][1], az = R.axis[link][2];
         const float wx = P[0] * ax + P[1] * ay + P[2] * az;
         const float wy = P[3] * ax + P[4] * ay + P[5] * az;
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, 
       enmax = fmaxf(enmax, fabsf(en[a]));
     }
     bool done = false;
-    if (start || (spd && En < E)) {
+    if (b >= 0 && (start || (spd && En < E))) {
       q = qn;
 #pragma unroll
       for (int t = 0; t < 12; ++t) P[t] = Pn[t];
@@ -251,7 +255,7 @@ __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, 
         mu = fmaxf(mu * 0.25f, 1e-10f);
         ++it;
       }
-    } else {
+    } else if (b >= 0) {
       mu *= 8.f;
       if (mu > 1e6f) done = true;  // gives up
       else ++it;
@@ -266,6 +270,9 @@ __global__ void __launch_bounds__(256, 2) k_ik(const KWorldDev* __restrict__ W, 
         if (A.iters) A.iters[b] = it;
       }
       b = -1;
+      mu = 1.f;
+#pragma unroll
+      for (int a = 0; a < M; ++a) e[a] = 0.1f;
     }
   }
 }
@@ -294,15 +301,17 @@ cudaError_t launch_ik(const KWorldDev* W, int robot, int B, float* q, const int*
   A.iters = iters;
   // one wave of blocks (2 of 8 warps per SM), each with its share of the
   // problems: the queue is the block's own, so calls on several streams do not
-  // share anything.  Fewer problems than groups: one each
-  const int threads = 256, groups = threads / 32 * (nlinks <= 8 ? 4 : (nlinks <= 16 ? 2 : 1));
-  const int share = (B + 2 * num_sms - 1) / (2 * num_sms);
-  A.per_block = share > groups ? share : groups;
+  // share anything.  (Fewer problems per warp than fit gain nothing even where
+  // warps are left over: 9,000 problems 377 us at 4 per warp, 433 us at 1;
+  // 554 problems 250 us either way.)
+  const int threads = 256;
+  A.per_block = (B + 2 * num_sms - 1) / (2 * num_sms);
   const int blocks = (B + A.per_block - 1) / A.per_block;
-  if (nlinks <= 8) {
+  const int width = nlinks <= 8 ? 8 : (nlinks <= 16 ? 16 : 32);
+  if (width == 8) {
     if (Rtarget) k_ik<6, 8><<<blocks, threads, 0, s>>>(W, A);
     else k_ik<3, 8><<<blocks, threads, 0, s>>>(W, A);
-  } else if (nlinks <= 16) {
+  } else if (width == 16) {
     if (Rtarget) k_ik<6, 16><<<blocks, threads, 0, s>>>(W, A);
     else k_ik<3, 16><<<blocks, threads, 0, s>>>(W, A);
   } else {
