@@ -226,6 +226,60 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
   return ncand + __popc(mk);
 }
 
+// Lower bound on the distance below two nodes of the trees, less every band a
+// comparison with m32 (1 + 2e-5) needs: placement dd of both sides, rounding,
+// and the width of the candidates' FP32 band.
+template <bool IDB>
+__device__ __forceinline__ float node_lb32(const MeshView& A, const MeshView& B, const float* TA, const float* TB,
+                                           const KNode& na, const KNode& nb, int nodeA, int nodeB, float dd)
+{
+  const Box32 BA = xform_box(TA, na.a, na.b);
+  Box32 BB;
+  if (IDB) {
+    BB.c = make_float3(nb.a.x, nb.a.y, nb.a.z);
+    BB.h = make_float3(nb.b.x, nb.b.y, nb.b.z);
+  } else {
+    BB = xform_box(TB, nb.a, nb.b);
+  }
+  const float slack = 4.f * kU * (fabsf(BA.c.x) + fabsf(BA.c.y) + fabsf(BA.c.z) + fabsf(BB.c.x) + fabsf(BB.c.y) +
+                                  fabsf(BB.c.z) + 1.f) +
+                      dd * 4.7321f + 1e-5f;
+  float lb = box_dist32(BA, BB.c, BB.h);
+  const float3 d = sub3(BA.c, BB.c);
+  const float n2 = dot3(d, d);
+  if (IDB) {
+    // the rotation-invariant sphere about A's node centre is tighter than the
+    // world box of a rotated node in most directions
+    const float gx = fmaxf(0.f, fabsf(d.x) - BB.h.x);
+    const float gy = fmaxf(0.f, fabsf(d.y) - BB.h.y);
+    const float gz = fmaxf(0.f, fabsf(d.z) - BB.h.z);
+    lb = fmaxf(lb, sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA));
+  } else {
+    lb = fmaxf(lb, sqrtf(d.x * d.x + d.y * d.y + d.z * d.z) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA) -
+                       __ldg(B.node_r + nodeB));
+  }
+  // separation along the line of centres: both boxes projected onto it
+  // (columns of T give the rotated box's half widths along d).  Boxes small
+  // against their distance are bounded almost exactly; the soft-min tests 28%
+  // fewer triangle pairs with it
+  if (n2 > 1e-12f) {
+    const float rn = rsqrtf(n2);
+    float w = fabsf(TA[0] * d.x + TA[3] * d.y + TA[6] * d.z) * na.b.x +
+              fabsf(TA[1] * d.x + TA[4] * d.y + TA[7] * d.z) * na.b.y +
+              fabsf(TA[2] * d.x + TA[5] * d.y + TA[8] * d.z) * na.b.z;
+    if (IDB)
+      w += fabsf(d.x) * BB.h.x + fabsf(d.y) * BB.h.y + fabsf(d.z) * BB.h.z;
+    else
+      w += fabsf(TB[0] * d.x + TB[3] * d.y + TB[6] * d.z) * nb.b.x +
+           fabsf(TB[1] * d.x + TB[4] * d.y + TB[7] * d.z) * nb.b.y +
+           fabsf(TB[2] * d.x + TB[5] * d.y + TB[8] * d.z) * nb.b.z;
+    // (the projections err by at most 4u |d| (|h| + |d|); 16u covers them
+    // and the normalisation)
+    lb = fmaxf(lb, (n2 - w) * rn - 16.f * kU * (n2 + w) * rn);
+  }
+  return lb - slack;
+}
+
 struct PairCnt {
   unsigned nodes = 0, tri = 0, fp64 = 0;  // per lane
 };
@@ -353,52 +407,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
       const int nodeA = (int)en.x, nodeB = (int)en.y;
       const KNode na = A.nodes[nodeA];
       const KNode nb = B.nodes[nodeB];
-      const Box32 BA = xform_box(TA, na.a, na.b);
-      Box32 BB;
-      if (IDB) {
-        BB.c = make_float3(nb.a.x, nb.a.y, nb.a.z);
-        BB.h = make_float3(nb.b.x, nb.b.y, nb.b.z);
-      } else {
-        BB = xform_box(TB, nb.a, nb.b);
-      }
-      const float slack = 4.f * kU * (fabsf(BA.c.x) + fabsf(BA.c.y) + fabsf(BA.c.z) + fabsf(BB.c.x) +
-                                      fabsf(BB.c.y) + fabsf(BB.c.z) + 1.f) +
-                          dd * 1.7321f;
-      float lb = box_dist32(BA, BB.c, BB.h);
-      if (IDB) {
-        // the rotation-invariant sphere about A's node centre is tighter than
-        // the world box of a rotated node in most directions
-        const float gx = fmaxf(0.f, fabsf(BA.c.x - BB.c.x) - BB.h.x);
-        const float gy = fmaxf(0.f, fabsf(BA.c.y - BB.c.y) - BB.h.y);
-        const float gz = fmaxf(0.f, fabsf(BA.c.z - BB.c.z) - BB.h.z);
-        lb = fmaxf(lb, sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA));
-      } else {
-        const float cx = BA.c.x - BB.c.x, cy = BA.c.y - BB.c.y, cz = BA.c.z - BB.c.z;
-        lb = fmaxf(lb, sqrtf(cx * cx + cy * cy + cz * cz) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA) -
-                           __ldg(B.node_r + nodeB));
-      }
-      // separation along the line of centres: both boxes projected onto it
-      // (columns of T give the rotated box's half widths along d).  Boxes
-      // small against their distance are bounded almost exactly; the soft-min
-      // tests 28% fewer triangle pairs with it
-      const float3 d = sub3(BA.c, BB.c);
-      const float n2 = dot3(d, d);
-      if (n2 > 1e-12f) {
-        const float rn = rsqrtf(n2);
-        float w = fabsf(TA[0] * d.x + TA[3] * d.y + TA[6] * d.z) * na.b.x +
-                  fabsf(TA[1] * d.x + TA[4] * d.y + TA[7] * d.z) * na.b.y +
-                  fabsf(TA[2] * d.x + TA[5] * d.y + TA[8] * d.z) * na.b.z;
-        if (IDB)
-          w += fabsf(d.x) * BB.h.x + fabsf(d.y) * BB.h.y + fabsf(d.z) * BB.h.z;
-        else
-          w += fabsf(TB[0] * d.x + TB[3] * d.y + TB[6] * d.z) * nb.b.x +
-               fabsf(TB[1] * d.x + TB[4] * d.y + TB[7] * d.z) * nb.b.y +
-               fabsf(TB[2] * d.x + TB[5] * d.y + TB[8] * d.z) * nb.b.z;
-        // (the projections err by at most 4u |d| (|h| + |d|); 16u covers them
-        // and the normalisation)
-        lb = fmaxf(lb, (n2 - w) * rn - 16.f * kU * (n2 + w) * rn);
-      }
-      if (lb - slack <= m32 * (1.f + 2e-5f) + 3.f * dd + 1e-5f) {
+      if (node_lb32<IDB>(A, B, TA, TB, na, nb, nodeA, nodeB, dd) <= m32 * (1.f + 2e-5f)) {
         const int cntA = f2i(na.b.w), cntB = f2i(nb.b.w);
         const int ia = f2i(na.a.w), ib = f2i(nb.a.w);
         if (cntA > 0 && cntB > 0) {
