@@ -1088,6 +1088,8 @@ __global__ void k_softmin_final(const double* wsum, const unsigned long long* mk
 // transforms.  One warp per configuration: FP32 traversal of each pair with
 // conservative pruning against the running upper bound of the minimum,
 // triangle pairs within the error band finalised in canonical FP64.
+constexpr int kSW = 2;  // warps per block of k_self_dist
+
 struct __align__(16) SelfDistSmem;
 __device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                              int lane, int i, int j);
@@ -1098,6 +1100,7 @@ struct __align__(16) SelfDistSmem {
   double T64[kMaxLinks][12];
   double q64[kMaxLinks];
   PairSmem P;                  // the current pair; P.b2 starts at the acceptance bound
+  float plb[kMaxLinks * (kMaxLinks - 1) / 2];  // lower bounds of the pairs still to evaluate
   double b2, bcp[3], bcq[3];  // best over the pairs so far: squared distance, closest points
   double bd;                   // its distance (the cutoff before any pair is found)
   int bi, bj;
@@ -1158,7 +1161,55 @@ __device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* _
   return sqrtf(bo) * (1.f + 1e-5f) + 2.f * (S.delta[i] + S.delta[j]) + 1e-6f;
 }
 
-__global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
+// Per-pair mode: every queried pair's own minimum, in order.
+__device__ __noinline__ void self_pairs(SelfDistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
+                                        const MeshView& M, const SelfDistArgs& A, int b, int lane, float fcut,
+                                        PairCnt& cnt)
+{
+  const int nl = R.nlinks, npair = nl * (nl - 1) / 2;
+  for (int k = lane; k < npair; k += 32) A.dpair[(size_t)b * npair + k] = -1.0;  // pairs not queried
+  __syncwarp();
+  const int nq = A.all_pairs ? npair : R.nqueries_self;
+#pragma unroll 1
+  for (int qi = 0; qi < nq; ++qi) {
+    int i, j;
+    if (A.all_pairs) {  // qi in upper-triangle order (0,1), (0,2), ..., (L-2, L-1)
+      i = 0;
+      int r = qi;
+      while (r >= nl - 1 - i) { r -= nl - 1 - i; ++i; }
+      j = i + 1 + r;
+    } else {
+      const uint32_t qw = __ldg(W->queries + R.query_off + R.nqueries_env + qi);
+      i = qw & 0xff;
+      j = (qw >> 8) & 0xff;
+    }
+    if (R.link_root[i] < 0 || R.link_root[j] < 0) continue;
+    float m32 = fminf(fcut, link_pair_seed(S, W, R, lane, i, j));
+    if (lane == 0) {
+      const double bb = kx_mul(A.cutoff, A.cutoff);
+      S.P.b2 = bb > 1e-300 ? bb : 1e-300;
+      S.P.bA = S.P.bB = INT_MAX;
+      S.P.have = 0;
+    }
+    int certA = -1;
+    const int r = pair_distance<false, true>(S.P, M, M, R.link_root[i], R.link_root[j], S.T[i], S.T[j], S.T64[i],
+                                             S.T64[j], S.delta[i] + S.delta[j], m32, certA, lane, cnt, [] {});
+    if (lane == 0) {
+      if (r == 2) set_status(W->status, KGPU_ERR_OVERFLOW);
+      A.dpair[(size_t)b * npair + i * nl - i * (i + 1) / 2 + (j - i - 1)] =
+          r == 1 ? 0.0 : (S.P.have ? kx_sqrt(S.P.b2) : A.cutoff);
+    }
+    __syncwarp();
+  }
+}
+
+// Pairs nearest first by their root boxes (all bounded at once, one per
+// lane): the first few set the bound that prunes the rest unseen, where the
+// (i, j) order evaluated most of a humanoid's 435.  The result is the
+// lexicographic minimum (distance, pair), whatever the order.  Blocks of two
+// warps, so that a costly configuration holds up one other at most.  8,192
+// humanoid configurations: 27.5 -> 5.96 ms (15.4 ms before this order).
+__global__ void __launch_bounds__(kSW * 32, 16 / kSW) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1168,9 +1219,10 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
   const KRobotDev& R = W->robots[A.robot];
   const int nl = R.nlinks;
   const float fcut = A.cutoff < 1e30 ? (float)A.cutoff * 1.000001f + 1e-7f : FLT_MAX;
-  const int nwarps = gridDim.x * kDW;
+  const bool per_pair = A.dpair != nullptr;
+  const int nwarps = gridDim.x * kSW;
 #pragma unroll 1
-  for (int b = blockIdx.x * kDW + warp; b < A.B; b += nwarps) {
+  for (int b = blockIdx.x * kSW + warp; b < A.B; b += nwarps) {
     const float qv = lane < nl ? __ldg(A.q + (size_t)b * nl + lane) : 0.f;
     if (__any_sync(0xffffffffu, lane < nl && !(fabsf(qv) < 1.0e6f))) {
       if (lane == 0) set_status(W->status, KGPU_ERR_NOT_FINITE);
@@ -1191,84 +1243,83 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_self_dist(const KWorldDev* __re
     }
     __syncwarp();
     warp_fk64(R, S.q64, S.T64, lane);
-    const bool per_pair = A.dpair != nullptr;
-    const int npair = nl * (nl - 1) / 2;
     if (per_pair) {
-      for (int k = lane; k < npair; k += 32) A.dpair[(size_t)b * npair + k] = -1.0;  // pairs not queried
-      __syncwarp();
+      self_pairs(S, W, R, M, A, b, lane, fcut, cnt);
+      continue;
     }
-    float m32 = fcut;  // upper bound on the minimum so far (warp-uniform)
-    bool contact = false;
-    const int nq = A.all_pairs ? npair : R.nqueries_self;
+    // lower bounds of all pairs from their root boxes, one pair per lane
+    const int nq = R.nqueries_self;
 #pragma unroll 1
-    for (int qi = 0; qi < nq && !contact; ++qi) {
-      int i, j;
-      if (A.all_pairs) {  // qi in upper-triangle order (0,1), (0,2), ..., (L-2, L-1)
-        i = 0;
-        int r = qi;
-        while (r >= nl - 1 - i) { r -= nl - 1 - i; ++i; }
-        j = i + 1 + r;
-      } else {
-        const uint32_t qw = __ldg(W->queries + R.query_off + R.nqueries_env + qi);
-        i = qw & 0xff;
-        j = (qw >> 8) & 0xff;
+    for (int k = lane; k < nq; k += 32) {
+      const uint32_t qw = __ldg(W->queries + R.query_off + R.nqueries_env + k);
+      const int i = qw & 0xff, j = (qw >> 8) & 0xff;
+      float lb = FLT_MAX;
+      if (R.link_root[i] >= 0 && R.link_root[j] >= 0)
+        lb = node_lb32<false>(M, M, S.T[i], S.T[j], W->lnodes[R.link_root[i]], W->lnodes[R.link_root[j]],
+                              R.link_root[i], R.link_root[j], S.delta[i] + S.delta[j]);
+      S.plb[k] = lb;
+    }
+    __syncwarp();
+    float m32 = fcut;  // upper bound on the minimum so far (warp-uniform)
+    int best = INT_MAX;  // position of the best pair in the (i, j) order
+#pragma unroll 1
+    for (;;) {
+      // the nearest pair by its boxes that can still win; once a contact is
+      // found, the first one in order before it (only an earlier contact can)
+      const bool contact = S.bd == 0.0 && best < INT_MAX;
+      const float lim = m32 * (1.f + 2e-5f);
+      float v = FLT_MAX;
+      int kq = INT_MAX;
+#pragma unroll 1
+      for (int k = lane; k < nq && !(contact && (k >= best || kq < INT_MAX)); k += 32) {
+        const float lb = S.plb[k];
+        if (lb <= lim && lb < v) {
+          v = contact ? -FLT_MAX : lb;
+          kq = k;
+        }
       }
-      if (R.link_root[i] < 0 || R.link_root[j] < 0) continue;
-      const float dd = S.delta[i] + S.delta[j];
-      bool pc = false;  // certified contact of this pair
-      if (per_pair) m32 = fcut;  // every pair on its own
-      // a pair without a running bound to prune with (the first, or every
-      // pair in per-pair mode) starts from a vertex-pair upper bound of its
-      // own distance (>= the running minimum including it, so the bound
-      // stays valid for the later pairs)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int ok = __shfl_xor_sync(0xffffffffu, kq, o);
+        if (ov < v || (ov == v && ok < kq)) { v = ov; kq = ok; }
+      }
+      if (kq == INT_MAX) break;
+      __syncwarp();
+      if (lane == 0) S.plb[kq] = FLT_MAX;
+      const uint32_t qw = __ldg(W->queries + R.query_off + R.nqueries_env + kq);
+      const int i = qw & 0xff, j = (qw >> 8) & 0xff;
+      // without a running bound to prune with, a vertex-pair bound of this pair
       if (m32 >= fcut) m32 = fminf(m32, link_pair_seed(S, W, R, lane, i, j));
       if (lane == 0) {
-        if (per_pair) S.bd = A.cutoff;
-        const double bb = kx_mul(S.bd, S.bd);
+        // below the best distance, or (an earlier pair) equal to it: 1e-15
+        // covers the squares whose root rounds to the same distance
+        double bb = kx_mul(S.bd, S.bd);
+        if (kq < best) bb = bb * (1.0 + 1e-15);
         S.P.b2 = bb > 1e-300 ? bb : 1e-300;
         S.P.bA = S.P.bB = INT_MAX;
         S.P.have = 0;
       }
       int certA = -1;
       const int r = pair_distance<false, true>(S.P, M, M, R.link_root[i], R.link_root[j], S.T[i], S.T[j], S.T64[i],
-                                               S.T64[j], dd, m32, certA, lane, cnt, [] {});
-      if (r == 2) {
-        if (lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
-      } else if (r == 1) {
-        pc = true;  // distance 0: no later pair can be smaller
-        if (lane == 0 && !per_pair) {
-          S.b2 = 0.0;
-          S.bd = 0.0;
+                                               S.T64[j], S.delta[i] + S.delta[j], m32, certA, lane, cnt, [] {});
+      if (r == 2 && lane == 0) set_status(W->status, KGPU_ERR_OVERFLOW);
+      const double dp = r == 1 ? 0.0 : (S.P.have ? kx_sqrt(S.P.b2) : DBL_MAX);
+      const bool first = best == INT_MAX;
+      if (r == 1 ? (first || S.bd > 0.0 || kq < best) : (dp < S.bd || (!first && dp == S.bd && kq < best))) {
+        __syncwarp();
+        if (lane == 0) {
+          S.b2 = r == 1 ? 0.0 : S.P.b2;
+          S.bd = dp;
           S.bi = i;
           S.bj = j;
+          for (int c = 0; c < 3; ++c) { S.bcp[c] = S.P.bcp[c]; S.bcq[c] = S.P.bcq[c]; }
         }
-        __syncwarp();
-      }
-      if (per_pair) {
-        if (lane == 0)
-          A.dpair[(size_t)b * npair + i * nl - i * (i + 1) / 2 + (j - i - 1)] =
-              pc ? 0.0 : (S.P.have ? kx_sqrt(S.P.b2) : A.cutoff);
-        __syncwarp();
-        continue;
-      }
-      // the pair replaces the best only with a strictly smaller distance
-      if (!pc && S.P.have) {
-        const double dp = kx_sqrt(S.P.b2);
-        if (dp < S.bd) {
-          __syncwarp();
-          if (lane == 0) {
-            S.b2 = S.P.b2;
-            S.bd = dp;
-            S.bi = i;
-            S.bj = j;
-            for (int c = 0; c < 3; ++c) { S.bcp[c] = S.P.bcp[c]; S.bcq[c] = S.P.bcq[c]; }
-          }
-        }
+        best = kq;
+        if (dp == 0.0) m32 = 0.f;
       }
       __syncwarp();
-      if (S.b2 == 0.0) contact = true;
     }
-    if (per_pair) continue;
     // ---- outputs and the gradient (FP64 transforms)
     const bool found = S.b2 < DBL_MAX;
     const double d = found ? kx_sqrt(S.b2) : A.cutoff;
@@ -1326,7 +1377,7 @@ cudaError_t dist_init()
     if (e != cudaSuccess) return e;
   }
   return cudaFuncSetAttribute(k_self_dist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sizeof(SelfDistSmem) * kDW));
+                              (int)(sizeof(SelfDistSmem) * kSW));
 }
 
 cudaError_t launch_distance(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int B, double cutoff,
@@ -1481,7 +1532,7 @@ cudaError_t launch_self_distance(const KWorldDev* Wd, int robot, const float* q,
                                  cudaStream_t s)
 {
   if (B <= 0) return cudaSuccess;
-  const size_t smem = sizeof(SelfDistSmem) * kDW;  // attribute set by dist_init()
+  const size_t smem = sizeof(SelfDistSmem) * kSW;  // attribute set by dist_init()
   SelfDistArgs A;
   A.robot = robot;
   A.q = q;
@@ -1493,8 +1544,8 @@ cudaError_t launch_self_distance(const KWorldDev* Wd, int robot, const float* q,
   A.grad = grad;
   A.dpair = dpair;
   A.all_pairs = dpair != nullptr && all_pairs != 0;
-  const int blocks = min((B + kDW - 1) / kDW, 4 * num_sms);
-  k_self_dist<<<blocks, kDW * 32, smem, s>>>(Wd, A);
+  const int blocks = min((B + kSW - 1) / kSW, 64 * num_sms);
+  k_self_dist<<<blocks, kSW * 32, smem, s>>>(Wd, A);
   return cudaGetLastError();
 }
 
