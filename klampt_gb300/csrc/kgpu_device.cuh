@@ -486,6 +486,82 @@ static __device__ __noinline__ int tri_overlap64(const double* P, const double* 
 constexpr unsigned kFeatAll = 0x7fffu;
 constexpr unsigned kFeatFlat = 1u << 15;  // a triangle without area: never taken as apart
 
+// kx_seg_seg with its divisions at three places instead of six: the same
+// operations on the same operands in every case.
+__device__ __forceinline__ double seg_seg64(const double* p1, const double* d1, const double* p2, const double* d2,
+                                            double* c1, double* c2)
+{
+  double r[3];
+  kx_sub3(p1, p2, r);
+  const double a = kx_dot3(d1, d1), e = kx_dot3(d2, d2), f = kx_dot3(d2, r), c = kx_dot3(d1, r), b = kx_dot3(d1, d2);
+  const bool pa = a <= 1e-300, pe = e <= 1e-300;  // a segment that is a point
+  double s = 0.0, t = 0.0;
+  if (!pa && !pe) {
+    const double den = kx_sub(kx_mul(a, e), kx_mul(b, b));
+    if (den > 0.0) s = kx_clamp01(kx_div(kx_sub(kx_mul(b, f), kx_mul(c, e)), den));
+  }
+  if (!pe) t = kx_div(pa ? f : kx_add(kx_mul(b, s), f), e);
+  const bool lo = t < 0.0, hi = t > 1.0;
+  if (pa) t = kx_clamp01(t);
+  else if (lo || hi || pe) {
+    s = kx_clamp01(kx_div(hi ? kx_sub(b, c) : -c, a));
+    t = hi ? 1.0 : 0.0;
+  }
+  double dd[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    c1[i] = kx_add(p1[i], kx_mul(d1[i], s));
+    c2[i] = kx_add(p2[i], kx_mul(d2[i], t));
+    dd[i] = kx_sub(c1[i], c2[i]);
+  }
+  return kx_dot3(dd, dd);
+}
+
+// kx_pt_tri with its divisions at two places instead of five: the first region
+// that holds is chosen, then its point is formed by the same operations.
+__device__ __forceinline__ double pt_tri64(const double* p, const double* a, const double* b, const double* c,
+                                           double* cp)
+{
+  double ab[3], ac[3], x[3];
+  kx_sub3(b, a, ab);
+  kx_sub3(c, a, ac);
+  kx_sub3(p, a, x);
+  const double d1 = kx_dot3(ab, x), d2 = kx_dot3(ac, x);
+  kx_sub3(p, b, x);
+  const double d3 = kx_dot3(ab, x), d4 = kx_dot3(ac, x);
+  kx_sub3(p, c, x);
+  const double d5 = kx_dot3(ab, x), d6 = kx_dot3(ac, x);
+  const double vc = kx_sub(kx_mul(d1, d4), kx_mul(d3, d2));
+  const double vb = kx_sub(kx_mul(d5, d2), kx_mul(d1, d6));
+  const double va = kx_sub(kx_mul(d3, d6), kx_mul(d5, d4));
+  const double e4 = kx_sub(d4, d3), e5 = kx_sub(d5, d6);
+  // 0: vertex a, 1: vertex b, 2: edge ab, 3: vertex c, 4: edge ac, 5: edge bc, 6: inside
+  const int g = d1 <= 0.0 && d2 <= 0.0 ? 0
+                : d3 >= 0.0 && d4 <= d3 ? 1
+                : vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0 ? 2
+                : d6 >= 0.0 && d5 <= d6 ? 3
+                : vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0 ? 4
+                : va <= 0.0 && e4 >= 0.0 && e5 >= 0.0 ? 5 : 6;
+  const bool point = g == 0 || g == 1 || g == 3;
+  double v = 0.0, w = 0.0;
+  if (!point) {
+    const double den = g == 2 ? kx_sub(d1, d3) : (g == 4 ? kx_sub(d2, d6) : (g == 5 ? kx_add(e4, e5)
+                                                                                     : kx_add(kx_add(va, vb), vc)));
+    v = kx_div(g == 2 ? d1 : (g == 4 ? d2 : (g == 5 ? e4 : vb)), den);
+    if (g == 6) w = kx_div(vc, den);
+  }
+  double dd[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double y = g == 1 || g == 5 ? b[i] : (g == 3 ? c[i] : a[i]);
+    if (!point) y = kx_add(y, kx_mul(g == 4 ? ac[i] : (g == 5 ? kx_sub(c[i], b[i]) : ab[i]), v));
+    if (g == 6) y = kx_add(y, kx_mul(ac[i], w));
+    cp[i] = y;
+    dd[i] = kx_sub(p[i], y);
+  }
+  return kx_dot3(dd, dd);
+}
+
 static __device__ __noinline__ double tri_dist2_masked64(const double* P, const double* Q, unsigned mask, bool apart,
                                                          double* cp, double* cq)
 {
@@ -508,7 +584,7 @@ static __device__ __noinline__ double tri_dist2_masked64(const double* P, const 
     const int k = __ffs(m) - 1, i = k / 3, j = k % 3;
     kx_sub3(p + 3 * (i == 2 ? 0 : i + 1), p + 3 * i, d1);
     kx_sub3(q + 3 * (j == 2 ? 0 : j + 1), q + 3 * j, d2);
-    const double d = kx_seg_seg(p + 3 * i, d1, q + 3 * j, d2, c, c2);
+    const double d = seg_seg64(p + 3 * i, d1, q + 3 * j, d2, c, c2);
     if (d < best) {
       best = d;
 #pragma unroll
@@ -521,7 +597,7 @@ static __device__ __noinline__ double tri_dist2_masked64(const double* P, const 
     const bool ofp = k < 3;  // a vertex of P against Q, or of Q against P
     const double* x = ofp ? p + 3 * k : q + 3 * (k - 3);
     const double* t3 = ofp ? q : p;
-    const double d = kx_pt_tri(x, t3, t3 + 3, t3 + 6, c);
+    const double d = pt_tri64(x, t3, t3 + 3, t3 + 6, c);
     if (d < best) {
       best = d;
 #pragma unroll

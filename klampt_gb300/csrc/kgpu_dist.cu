@@ -142,6 +142,7 @@ __device__ __noinline__ float pair_seed(DistSmem& S, const KWorldDev* __restrict
   const int vf = R.link_vert_first[l], vc = R.link_vert_count[l];
   float bd = FLT_MAX;
   float3 bv = make_float3(ob.a.x, ob.a.y, ob.a.z);
+#pragma unroll 2
   for (int v = lane; v < vc; v += 32) {
     const float4 x = __ldg(W->lvert32 + vf + v);
     const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
@@ -156,6 +157,7 @@ __device__ __noinline__ float pair_seed(DistSmem& S, const KWorldDev* __restrict
   bv = make_float3(__shfl_sync(0xffffffffu, bv.x, src), __shfl_sync(0xffffffffu, bv.y, src),
                    __shfl_sync(0xffffffffu, bv.z, src));
   float bo = FLT_MAX;
+#pragma unroll 2
   for (int t = lane; t < fc; t += 32) {
     const float4 y = __ldg(W->etri32 + 3 * (size_t)(ff + t));
     const float dx = y.x - bv.x, dy = y.y - bv.y, dz = y.z - bv.z;
@@ -216,6 +218,124 @@ struct PairOut {
   float dir[3];
 };
 
+// The deepest vertex of link l inside the convex object o (canonical FP64
+// depth, ties to the smaller vertex) and the face it is nearest to; 0 and no
+// vertex when none is strictly inside.  Out of line: contacts are rare in some
+// workloads, and its code is larger than the traversal's.
+__device__ __noinline__ double link_depth(DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
+                                          double (*T64)[12], int& fk64, int lane, int l, int o, float dd, int& vbest,
+                                          int& fbest)
+{
+  const float* TA = S.T[l];
+  double depth = 0.0;
+  // deepest link vertex inside the convex object
+  const int vf = R.link_vert_first[l], vc = R.link_vert_count[l];
+  const KNode ob = W->enodes[W->obj_root[o]];
+  const float tolb = dd + 8.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + 1.f);
+  const int ff = W->obj_leaf_first[o], fc = W->obj_leaf_count[o];
+  const float ed = depth_band(ob, dd);
+  float lmax = -FLT_MAX;
+  // pass 1: FP32 depths, lane-local maximum.  Each lane also keeps the (at
+  // most two) vertices whose pass-1 value lies within 2 ed of its running
+  // maximum: pass 1's value bounds a vertex's full FP32 minimum from
+  // above, and the global maximum is at least the lane's, so every vertex
+  // that pass 2 can accept is among them, unless more than two qualified
+  // (then the lane rescans all of its vertices)
+  int cv0 = 0, cv1 = 0, nc = 0;
+  float cd0 = 0.f, cd1 = 0.f;
+  bool rescan = false;
+#pragma unroll 1
+  for (int v = lane; v < vc; v += 32) {
+    const float4 x = __ldg(W->lvert32 + vf + v);
+    const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
+    if (fabsf(w.x - ob.a.x) > ob.b.x + tolb || fabsf(w.y - ob.a.y) > ob.b.y + tolb ||
+        fabsf(w.z - ob.a.z) > ob.b.z + tolb)
+      continue;
+    // a vertex stops counting once it is no deeper than the deepest so far
+    // (or outside the band): its final minimum can only be lower
+    const float stop = fmaxf(lmax, -ed);
+    float dmin = FLT_MAX;
+#pragma unroll 1
+    for (int f = ff; f < ff + fc && dmin > stop; ++f) {
+      const float4 pl = __ldg(W->eface32 + f);
+      dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
+    }
+    lmax = fmaxf(lmax, dmin);
+    const float thr = lmax - 2.f * ed;
+    if (dmin > -ed && dmin >= thr) {
+      if (nc == 2 && cd1 < thr) nc = 1;
+      if (nc >= 1 && cd0 < thr) {
+        if (nc == 2) { cv0 = cv1; cd0 = cd1; }
+        --nc;
+      }
+      if (nc == 0) { cv0 = v; cd0 = dmin; nc = 1; }
+      else if (nc == 1) { cv1 = v; cd1 = dmin; nc = 2; }
+      else rescan = true;
+    }
+  }
+  const float gmax = -warp_min(-lmax);
+  if (gmax > -ed) {
+    dist_fk64(S, R, T64, lane, fk64);
+    // pass 2: FP64 depth of every vertex within the band of the deepest
+    double bd = 0.0;
+    int bv = INT_MAX, bf = -1;
+    auto depth64 = [&](int v) {
+      const float4 x = __ldg(W->lvert32 + vf + v);
+      const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
+      if (fabsf(w.x - ob.a.x) > ob.b.x + tolb || fabsf(w.y - ob.a.y) > ob.b.y + tolb ||
+          fabsf(w.z - ob.a.z) > ob.b.z + tolb)
+        return;
+      const float stop = fmaxf(gmax - 2.f * ed, -ed);
+      float dmin = FLT_MAX;
+#pragma unroll 1
+      for (int f = ff; f < ff + fc && dmin >= stop; ++f) {
+        const float4 pl = __ldg(W->eface32 + f);
+        dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
+      }
+      if (dmin < gmax - 2.f * ed || dmin <= -ed) return;
+      double w64[3];
+      kx_xform_point(T64[l], W->lvert64 + 3 * (size_t)(vf + v), w64);
+      double dm = DBL_MAX;
+      int fm = -1, fo = INT_MAX;
+#pragma unroll 1
+      for (int f = ff; f < ff + fc; ++f) {
+        // (the nearest face in FP64 lies within the band of the nearest in FP32)
+        const float4 pl32 = __ldg(W->eface32 + f);
+        if (pl32.w - (pl32.x * w.x + pl32.y * w.y + pl32.z * w.z) > dmin + 2.f * ed) continue;
+        const double* pl = W->eface64 + 4 * (size_t)f;
+        const double dep = kx_sub(pl[3], kx_dot3(pl, w64));
+        const int orig = W->etri_orig[f];
+        if (dep < dm || (dep == dm && orig < fo)) { dm = dep; fm = f; fo = orig; }
+      }
+      if (dm > bd || (dm == bd && dm > 0.0 && v < bv)) { bd = dm; bv = v; bf = fm; }
+    };
+    if (rescan) {
+#pragma unroll 1
+      for (int v = lane; v < vc; v += 32) depth64(v);
+    } else {
+      if (nc >= 1 && cd0 >= gmax - 2.f * ed) depth64(cv0);
+      if (nc >= 2 && cd1 >= gmax - 2.f * ed) depth64(cv1);
+    }
+    // warp maximum of (depth, -vertex)
+    double wd = bd;
+    int wv = bd > 0.0 ? bv : INT_MAX, wf = bf, src = lane;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const double od = __shfl_xor_sync(0xffffffffu, wd, off);
+      const int ov = __shfl_xor_sync(0xffffffffu, wv, off);
+      const int ofc = __shfl_xor_sync(0xffffffffu, wf, off);
+      const int os = __shfl_xor_sync(0xffffffffu, src, off);
+      if (od > wd || (od == wd && (ov < wv || (ov == wv && os < src)))) { wd = od; wv = ov; wf = ofc; src = os; }
+    }
+    if (wd > 0.0) {
+      depth = wd;
+      vbest = wv;
+      fbest = wf;
+    }
+  }
+  return depth;
+}
+
 // Signed distance of (link l, object o) below `bound` (found = d < bound).
 __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                        double (*T64)[12], int& fk64, int lane, int l, int o, double bound,
@@ -262,110 +382,7 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
   // ---- surfaces meet
   int vbest = -1, fbest = -1;
   double depth = 0.0;
-  if (W->obj_convex[o]) {
-    // deepest link vertex inside the convex object
-    const int vf = R.link_vert_first[l], vc = R.link_vert_count[l];
-    const KNode ob = W->enodes[W->obj_root[o]];
-    const float tolb = dl + de + 8.f * kU * (fabsf(ob.a.x) + fabsf(ob.a.y) + fabsf(ob.a.z) + 1.f);
-    const int ff = W->obj_leaf_first[o], fc = W->obj_leaf_count[o];
-    const float ed = depth_band(ob, dl + de);
-    float lmax = -FLT_MAX;
-    // pass 1: FP32 depths, lane-local maximum.  Each lane also keeps the (at
-    // most two) vertices whose pass-1 value lies within 2 ed of its running
-    // maximum: pass 1's value bounds a vertex's full FP32 minimum from
-    // above, and the global maximum is at least the lane's, so every vertex
-    // that pass 2 can accept is among them, unless more than two qualified
-    // (then the lane rescans all of its vertices)
-    int cv0 = 0, cv1 = 0, nc = 0;
-    float cd0 = 0.f, cd1 = 0.f;
-    bool rescan = false;
-#pragma unroll 1
-    for (int v = lane; v < vc; v += 32) {
-      const float4 x = __ldg(W->lvert32 + vf + v);
-      const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
-      if (fabsf(w.x - ob.a.x) > ob.b.x + tolb || fabsf(w.y - ob.a.y) > ob.b.y + tolb ||
-          fabsf(w.z - ob.a.z) > ob.b.z + tolb)
-        continue;
-      // a vertex stops counting once it is no deeper than the deepest so far
-      // (or outside the band): its final minimum can only be lower
-      const float stop = fmaxf(lmax, -ed);
-      float dmin = FLT_MAX;
-#pragma unroll 1
-      for (int f = ff; f < ff + fc && dmin > stop; ++f) {
-        const float4 pl = __ldg(W->eface32 + f);
-        dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
-      }
-      lmax = fmaxf(lmax, dmin);
-      const float thr = lmax - 2.f * ed;
-      if (dmin > -ed && dmin >= thr) {
-        if (nc == 2 && cd1 < thr) nc = 1;
-        if (nc >= 1 && cd0 < thr) {
-          if (nc == 2) { cv0 = cv1; cd0 = cd1; }
-          --nc;
-        }
-        if (nc == 0) { cv0 = v; cd0 = dmin; nc = 1; }
-        else if (nc == 1) { cv1 = v; cd1 = dmin; nc = 2; }
-        else rescan = true;
-      }
-    }
-    const float gmax = -warp_min(-lmax);
-    if (gmax > -ed) {
-      dist_fk64(S, R, T64, lane, fk64);
-      // pass 2: FP64 depth of every vertex within the band of the deepest
-      double bd = 0.0;
-      int bv = INT_MAX, bf = -1;
-      auto depth64 = [&](int v) {
-        const float4 x = __ldg(W->lvert32 + vf + v);
-        const float3 w = xform32(TA, make_float3(x.x, x.y, x.z));
-        if (fabsf(w.x - ob.a.x) > ob.b.x + tolb || fabsf(w.y - ob.a.y) > ob.b.y + tolb ||
-            fabsf(w.z - ob.a.z) > ob.b.z + tolb)
-          return;
-        const float stop = fmaxf(gmax - 2.f * ed, -ed);
-        float dmin = FLT_MAX;
-#pragma unroll 1
-        for (int f = ff; f < ff + fc && dmin >= stop; ++f) {
-          const float4 pl = __ldg(W->eface32 + f);
-          dmin = fminf(dmin, pl.w - (pl.x * w.x + pl.y * w.y + pl.z * w.z));
-        }
-        if (dmin < gmax - 2.f * ed || dmin <= -ed) return;
-        double w64[3];
-        kx_xform_point(T64[l], W->lvert64 + 3 * (size_t)(vf + v), w64);
-        double dm = DBL_MAX;
-        int fm = -1, fo = INT_MAX;
-#pragma unroll 1
-        for (int f = ff; f < ff + fc; ++f) {
-          const double* pl = W->eface64 + 4 * (size_t)f;
-          const double dep = kx_sub(pl[3], kx_dot3(pl, w64));
-          const int orig = W->etri_orig[f];
-          if (dep < dm || (dep == dm && orig < fo)) { dm = dep; fm = f; fo = orig; }
-        }
-        if (dm > bd || (dm == bd && dm > 0.0 && v < bv)) { bd = dm; bv = v; bf = fm; }
-      };
-      if (rescan) {
-#pragma unroll 1
-        for (int v = lane; v < vc; v += 32) depth64(v);
-      } else {
-        if (nc >= 1 && cd0 >= gmax - 2.f * ed) depth64(cv0);
-        if (nc >= 2 && cd1 >= gmax - 2.f * ed) depth64(cv1);
-      }
-      // warp maximum of (depth, -vertex)
-      double wd = bd;
-      int wv = bd > 0.0 ? bv : INT_MAX, wf = bf, src = lane;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double od = __shfl_xor_sync(0xffffffffu, wd, off);
-        const int ov = __shfl_xor_sync(0xffffffffu, wv, off);
-        const int ofc = __shfl_xor_sync(0xffffffffu, wf, off);
-        const int os = __shfl_xor_sync(0xffffffffu, src, off);
-        if (od > wd || (od == wd && (ov < wv || (ov == wv && os < src)))) { wd = od; wv = ov; wf = ofc; src = os; }
-      }
-      if (wd > 0.0) {
-        depth = wd;
-        vbest = wv;
-        fbest = wf;
-      }
-    }
-  }
+  if (W->obj_convex[o]) depth = link_depth(S, W, R, T64, fk64, lane, l, o, dl + de, vbest, fbest);
   if (vbest >= 0) {
     double w64[3];
     kx_xform_point(T64[l], W->lvert64 + 3 * (size_t)(R.link_vert_first[l] + vbest), w64);
@@ -581,6 +598,19 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     if (MODE == 0 || MODE == 1) {
       // ---- minimum over pairs, iterative deepening of the search bound
       double best = A.cutoff;
+      // its FP32 neighbours for the comparisons of the pair loops (an FP64 one
+      // costs the SM as much as 40 of FP32): rounded up, the reach of a box
+      // bound (boxes bound the unsigned distance: a pair can be negative only
+      // when its boxes meet), and whether the rounding was exact
+      float best_up, reach;
+      bool best_exact;
+      auto set_best = [&](double d) {
+        best = d;
+        best_up = __double2float_ru(d);
+        best_exact = (double)best_up == d;
+        reach = fmaxf(best_up, 0.f) * 1.00001f + 1e-6f;
+      };
+      set_best(A.cutoff);
       int bl = -1, bo = -1;
       PairOut bp;
       bp.found = 0;
@@ -605,7 +635,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
           const int k = __shfl_sync(0xffffffffu, idx, owner);
           if (lane == 0) S.plb[k] = FLT_MAX;
           __syncwarp();
-          if (vm > (float)fmax(best, 0.0) * 1.00001f + 1e-6f) break;
+          if (vm > reach) break;
           const int o = S.pobj[k], l = S.plink[k];
           // a pair cannot go below 0 unless its object is convex, and then
           // not below minus the smallest half-extent of the object's box
@@ -615,13 +645,11 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
           // go below minus the depth of the link's deepest vertex in it
           if (bl >= 0) {
             const bool convex = W->obj_convex[o] != 0, tie = l < bl || (l == bl && o < bo);
-            const double dlow = convex ? -(double)fminf(fminf(W->enodes[W->obj_root[o]].b.x,
-                                                              W->enodes[W->obj_root[o]].b.y),
-                                                        W->enodes[W->obj_root[o]].b.z)
-                                       : 0.0;
-            if (dlow > best || (dlow == best && !tie)) continue;
-            if (convex && best <= 0.0 && !(best == 0.0 && tie) &&
-                !may_be_deeper(S, W, R, lane, l, o, (float)-best))
+            const float4 oh = W->enodes[W->obj_root[o]].b;
+            const float dlow = convex ? -fminf(fminf(oh.x, oh.y), oh.z) : 0.f;
+            if (dlow > best_up || (dlow == best_up && !(best_exact && tie))) continue;
+            if (convex && best_up <= 0.f && !(best == 0.0 && tie) &&
+                !may_be_deeper(S, W, R, lane, l, o, -best_up))
               continue;
           }
           PairOut po;
@@ -629,7 +657,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
           eval_pair(S, W, R, T64, fk64, lane, l, o, nextafter(best, 1e300), po, cnt,
                     bl < 0 ? pair_seed(S, W, R, lane, l, o) : FLT_MAX);
           if (po.found && (po.d < best || (po.d == best && (l < bl || (l == bl && o < bo))))) {
-            best = po.d;
+            set_best(po.d);
             bl = l;
             bo = o;
             bp = po;
@@ -647,9 +675,6 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
             if (lane == 0) S.gstack[0] = (uint32_t)W->group_root[g];
             __syncwarp();
             while (top > 0) {
-              // box bounds limit the unsigned distance: a pair can be
-              // negative only when its boxes meet, hence max(best, 0)
-              const float reach = (float)fmax(best, 0.0) * 1.00001f + 1e-6f;
               np = gather_objects(S, W, R, lane, l, fminf(bound, reach), lower, np, top);
               if (top > 0) {
                 // list full: evaluate what it holds, then keep gathering

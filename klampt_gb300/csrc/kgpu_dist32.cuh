@@ -101,21 +101,24 @@ done:
   return dot3(dd, dd);
 }
 
-// squared distance of two separated triangles: 9 edge-edge + 6 vertex-face
-static __device__ float tri_dist2_32(const float3* P, const float3* Q)
+// squared distance of two separated triangles: 9 edge-edge + 6 vertex-face.
+// The vertices come by value: through pointers they live in local memory, which
+// the loops' selections then read over and over (the distance kernels' L1, cut
+// short by their shared memory, missed 4 of 5 of those loads).
+static __device__ __noinline__ float tri_dist2_32(float3 P0, float3 P1, float3 P2, float3 Q0, float3 Q1, float3 Q2)
 {
   float best = FLT_MAX;
 #pragma unroll 1
   for (int k = 0; k < 9; ++k) {
     const int i = k / 3, j = k % 3;
-    const float3 pa = sel3(i, P[0], P[1], P[2]), pb = sel3(i == 2 ? 0 : i + 1, P[0], P[1], P[2]);
-    const float3 qa = sel3(j, Q[0], Q[1], Q[2]), qb = sel3(j == 2 ? 0 : j + 1, Q[0], Q[1], Q[2]);
+    const float3 pa = sel3(i, P0, P1, P2), pb = sel3(i == 2 ? 0 : i + 1, P0, P1, P2);
+    const float3 qa = sel3(j, Q0, Q1, Q2), qb = sel3(j == 2 ? 0 : j + 1, Q0, Q1, Q2);
     best = fminf(best, seg_seg2_32(pa, sub3(pb, pa), qa, sub3(qb, qa)));
   }
 #pragma unroll 1
   for (int k = 0; k < 3; ++k) {
-    best = fminf(best, pt_tri2_32(sel3(k, P[0], P[1], P[2]), Q[0], Q[1], Q[2]));
-    best = fminf(best, pt_tri2_32(sel3(k, Q[0], Q[1], Q[2]), P[0], P[1], P[2]));
+    best = fminf(best, pt_tri2_32(sel3(k, P0, P1, P2), Q0, Q1, Q2));
+    best = fminf(best, pt_tri2_32(sel3(k, Q0, Q1, Q2), P0, P1, P2));
   }
   return best;
 }
@@ -143,14 +146,15 @@ static __device__ float tri_dist2_32(const float3* P, const float3* Q)
 // kFeatFlat is set when a triangle has no area: the canonical overlap test can
 // report a contact of such triangles that are apart (its axes vanish), so the
 // pair is left to the whole canonical function.
-static __device__ __noinline__ unsigned tri_feature_mask32(const float3* P, const float3* Q, float thr2)
+static __device__ __noinline__ unsigned tri_feature_mask32(float3 P0, float3 P1, float3 P2, float3 Q0, float3 Q1,
+                                                              float3 Q2, float thr2)
 {
   unsigned mask = 0;
 #pragma unroll 1
   for (int k = 0; k < 9; ++k) {
     const int i = k / 3, j = k % 3;
-    const float3 pa = sel3(i, P[0], P[1], P[2]), pb = sel3(i == 2 ? 0 : i + 1, P[0], P[1], P[2]);
-    const float3 qa = sel3(j, Q[0], Q[1], Q[2]), qb = sel3(j == 2 ? 0 : j + 1, Q[0], Q[1], Q[2]);
+    const float3 pa = sel3(i, P0, P1, P2), pb = sel3(i == 2 ? 0 : i + 1, P0, P1, P2);
+    const float3 qa = sel3(j, Q0, Q1, Q2), qb = sel3(j == 2 ? 0 : j + 1, Q0, Q1, Q2);
     const float3 d1 = sub3(pb, pa), d2 = sub3(qb, qa);
     const float a = dot3(d1, d1), e = dot3(d2, d2), b = dot3(d1, d2);
     if (!(a * e - b * b >= 1e-3f * a * e) || !(seg_seg2_32(pa, d1, qa, d2) > thr2)) mask |= 1u << k;
@@ -158,7 +162,7 @@ static __device__ __noinline__ unsigned tri_feature_mask32(const float3* P, cons
 #pragma unroll 1
   for (int t = 0; t < 2; ++t) {
     // t = 0: vertices of P against Q, t = 1: vertices of Q against P
-    const float3 a = t ? P[0] : Q[0], b = t ? P[1] : Q[1], c = t ? P[2] : Q[2];
+    const float3 a = t ? P0 : Q0, b = t ? P1 : Q1, c = t ? P2 : Q2;
     const float3 ab = sub3(b, a), ac = sub3(c, a), bc = sub3(c, b);
     const float3 n = cross3(ab, ac);
     const float L2 = fmaxf(dot3(ab, ab), fmaxf(dot3(ac, ac), dot3(bc, bc)));
@@ -167,7 +171,7 @@ static __device__ __noinline__ unsigned tri_feature_mask32(const float3* P, cons
     if (!(n2 >= 1e-8f * L2 * L2)) mask |= kFeatFlat;
 #pragma unroll 1
     for (int k = 0; k < 3; ++k) {
-      const float3 p = t ? sel3(k, Q[0], Q[1], Q[2]) : sel3(k, P[0], P[1], P[2]);
+      const float3 p = t ? sel3(k, Q0, Q1, Q2) : sel3(k, P0, P1, P2);
       if (thin || !(pt_tri2_32(p, a, b, c) > thr2)) mask |= 1u << (9 + 3 * t + k);
     }
   }

@@ -153,7 +153,8 @@ __device__ __noinline__ int pair_flush(PairSmem& S, const MeshView& A, const Mes
       float3 P32[3], Q32[3];
       place32<false>(A, TA, tA, P32);
       place32<IDB>(B, TB, tB, Q32);
-      const unsigned mask = tri_feature_mask32(P32, Q32, feature_thr2(P32, Q32, m32, dd));
+      const unsigned mask = tri_feature_mask32(P32[0], P32[1], P32[2], Q32[0], Q32[1], Q32[2],
+                                               feature_thr2(P32, Q32, m32, dd));
       d2 = tri_dist2_masked64(P, Q, mask, S.candS[k] != 0, cp, cq);
       oa = A.orig[tA];
       ob = B.orig[tB];
@@ -200,11 +201,12 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
       place32<false>(A, TA, tA, P);
       place32<IDB>(B, TB, tB, Q);
       e = dd + 128.f * kU * tri_span(P, Q) + 1e-8f;
-      if (!tri_separated32(P, Q, dd, 0.f)) {
+      // (a positive lower bound, bands included, has them apart already)
+      if (!(S.fullL[k] > 0.f) && !tri_separated32(P, Q, dd, 0.f)) {
         d32 = 0.f;
         if (CERT) certain = tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd);
       } else {
-        d32 = sqrtf(tri_dist2_32(P, Q));
+        d32 = sqrtf(tri_dist2_32(P[0], P[1], P[2], Q[0], Q[1], Q[2]));
       }
     }
   }
@@ -399,12 +401,12 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
     if (have) en = S.stack[top - 1 - lane];
     __syncwarp();
     top -= n;
+    const int nodeA = (int)en.x, nodeB = (int)en.y;
     int outcome = 0;
     uint2 c0 = make_uint2(0, 0), c1 = make_uint2(0, 0);
     uint32_t jA = 0, jB = 0;
     cnt.nodes += have ? 1 : 0;
     if (have) {
-      const int nodeA = (int)en.x, nodeB = (int)en.y;
       const KNode na = A.nodes[nodeA];
       const KNode nb = B.nodes[nodeB];
       if (node_lb32<IDB>(A, B, TA, TB, na, nb, nodeA, nodeB, dd) <= m32 * (1.f + 2e-5f)) {
