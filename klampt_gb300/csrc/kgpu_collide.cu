@@ -50,6 +50,7 @@ constexpr int kGrab = 2;  // items taken from the queue per atomic
 constexpr int kWarps = 8; // warps per block
 constexpr int kMaxChunk = 64;  // most consecutive edge steps per work item
 constexpr int kDefaultChunk = 16;
+constexpr int kSmallEdges = 512;  // edges up to which a batch takes the SMALL kernel
 constexpr int kTailItemsPerWarp = 2;  // single-step rounds once fewer items than this per warp remain
 
 enum Mode { MODE_CONFIGS = 0, MODE_FEASIBLE = 1, MODE_EDGES = 2 };
@@ -198,7 +199,7 @@ __device__ __forceinline__ uint2 make_entry(int nodeA, int la, int tgt, int node
 // kernel keeps that kernel's hot loop in the instruction cache.  A contact
 // at step g clears bit g of `live` (edge steps: bits g and above, later
 // steps need no decision).  Returns the steps found in contact.
-template <bool FP64, bool EDGES>
+template <bool FP64, bool EDGES, bool SMALL>
 __device__ __noinline__ unsigned run_jobs(WarpSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                           int njobs, int lane, double (*T64)[12], int& fk64, const EngineArgs& A,
                                           Cnt& cnt, unsigned live, int lgL)
@@ -206,6 +207,13 @@ __device__ __noinline__ unsigned run_jobs(WarpSmem& S, const KWorldDev* __restri
   const int lmask = (1 << lgL) - 1;
   constexpr bool seq = EDGES;
   unsigned hits = 0;
+  if (SMALL) {
+    // with every step of an edge in work at once, those after its first
+    // contact (the costliest: the deepest contacts) stop when it is known
+    int fh = 0;
+    if (lane == 0) fh = *((volatile int*)(A.first_hit + S.item_id));
+    if (__shfl_sync(0xffffffffu, fh, 0) <= S.item_k) return 0;
+  }
   // exclusive prefix over job sizes
   uint32_t carry = 0;
 #pragma unroll 1
@@ -494,7 +502,7 @@ __device__ __noinline__ void restore_half(WarpSmem& S, const uint2* spill, int s
 // later steps).  Returns the steps found in contact (bits 0..3: a group has
 // at most 32 / 8 steps), plus kTrOverflow when the spill area ran out.
 // Warp-uniform control flow.
-template <bool FP64, bool EDGES, bool STAGE = false>
+template <bool FP64, bool EDGES, bool STAGE = false, bool SMALL = false>
 __device__ __noinline__ unsigned traverse(WarpSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                           int qbase, int qcount, int lane, uint2* spill, int spill_cap,
                                           double (*T64)[12], int& fk64, const EngineArgs& A, int job_flush,
@@ -574,7 +582,7 @@ __device__ __noinline__ unsigned traverse(WarpSmem& S, const KWorldDev* __restri
       }
     }
     if (njobs >= job_flush || (top == 0 && njobs > 0)) {
-      const unsigned r = run_jobs<FP64, EDGES>(S, W, R, njobs, lane, T64, fk64, A, cnt, live, lgL);
+      const unsigned r = run_jobs<FP64, EDGES, SMALL>(S, W, R, njobs, lane, T64, fk64, A, cnt, live, lgL);
       hits |= r & 0xffffu;
       live = r >> 16;
       __syncwarp();
@@ -639,7 +647,12 @@ __device__ __noinline__ unsigned traverse(WarpSmem& S, const KWorldDev* __restri
 // pairs are common and an inline FP64 contact ends an item early) or as the
 // fallback after a main pass whose list overflowed (otherwise it returns at
 // once); its verdicts overwrite the main pass's.
-template <int MINB, bool FP64, bool EDGES, bool STAGE = false>
+// SMALL (edges): batches of few edges, whose steps are in work side by side;
+// those after an edge's first contact stop when it is known.  An instantiation
+// of its own, because the check costs large batches 3% by its mere presence
+// (16,384 edges 1,620 -> 1,672 us).  24 edges 231 -> 176 us, 60 edges 272 ->
+// 208 us, 200 edges 194 -> 173 us.
+template <int MINB, bool FP64, bool EDGES, bool STAGE = false, bool SMALL = false>
 __global__ void __launch_bounds__(kWarps * 32, MINB)
     k_engine(const KWorldDev* __restrict__ W, const EngineArgs A)
 {
@@ -684,7 +697,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
   const int total = EDGES ? A.meta[1] : (A.perm ? A.meta[0] : (A.B + Gcfg - 1) / Gcfg);
   const int maxn = EDGES ? A.meta[0] : 0;  // last round index
   const int grab = A.grab >= 1 && A.grab <= 16 ? A.grab : kGrab;
-  const int job_flush = A.job_flush >= 8 && A.job_flush <= kJobCap - 32 ? A.job_flush : kJobCap - 32;
+  const int job_flush_opt = A.job_flush >= 8 && A.job_flush <= kJobCap - 32 ? A.job_flush : kJobCap - 32;
   const int chunk = A.chunk >= 1 && A.chunk <= kMaxChunk ? A.chunk : 1;
   const int nchunked = EDGES ? A.meta[2] : 0;
   const int split = EDGES ? A.meta[3] : 0;
@@ -696,6 +709,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
   // 231 us, 8 edges 211 -> 183 us
   const bool deal = (unsigned)total <= gridDim.x * (unsigned)kWarps;
   bool dealt = false;
+  // jobs tested earlier: a contact found sooner ends the item, and lanes are
+  // idle anyway (500 feasibility checks 247 -> 241 us, 24 edges 231 -> 217 us)
+  const int job_flush = deal ? min(job_flush_opt, 32) : job_flush_opt;
 
 #pragma unroll 1
   for (;;) {
@@ -858,15 +874,15 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
           // drain per group instead of two)
           const int nq = R.nqueries_env + R.nqueries_self;
           if (nq > 0)
-            env_hits = traverse<FP64, EDGES, STAGE>(S, W, R, R.query_off, nq, lane, spill, spill_cap, T64, fk64,
+            env_hits = traverse<FP64, EDGES, STAGE, SMALL>(S, W, R, R.query_off, nq, lane, spill, spill_cap, T64, fk64,
                                                     A, job_flush, cnt, all, warp, B, 0, live, lgL, nstage);
         } else {
           // configurations report the environment and self verdicts apart
           if (A.env_hit != nullptr && R.nqueries_env > 0)
-            env_hits = traverse<FP64, EDGES, STAGE>(S, W, R, R.query_off, R.nqueries_env, lane, spill, spill_cap,
+            env_hits = traverse<FP64, EDGES, STAGE, SMALL>(S, W, R, R.query_off, R.nqueries_env, lane, spill, spill_cap,
                                                     T64, fk64, A, job_flush, cnt, all, warp, B, 0, live, lgL, nstage);
           if (A.self_hit != nullptr && R.nqueries_self > 0)
-            self_hits = traverse<FP64, EDGES, STAGE>(S, W, R, R.query_off + R.nqueries_env, R.nqueries_self, lane,
+            self_hits = traverse<FP64, EDGES, STAGE, SMALL>(S, W, R, R.query_off + R.nqueries_env, R.nqueries_self, lane,
                                                      spill, spill_cap, T64, fk64, A, job_flush, cnt, all, warp, B, 0,
                                                      live, lgL, nstage);
         }
@@ -929,7 +945,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
         if (live != 0) {
           int fk64 = 0;
           const bool self = ((S.stack[0].y >> 25) & 63u) < 32u;
-          const unsigned hits = traverse<FP64, EDGES, STAGE>(S, W, R, 0, 0, lane, spill, spill_cap, T64, fk64, A,
+          const unsigned hits = traverse<FP64, EDGES, STAGE, SMALL>(S, W, R, 0, 0, lane, spill, spill_cap, T64, fk64, A,
                                                              job_flush, cnt, all, warp, B, S.don_top, live, lgL,
                                                              nstage);
           if (lane == 0) {
@@ -1615,10 +1631,10 @@ __global__ void k_jacobian(const KWorldDev* __restrict__ W, int robot, const flo
 template <bool STAGE>
 constexpr size_t engine_smem() { return STAGE ? kStageOffset + sizeof(KNode) * kStageNodes : kBlockSmem; }
 
-template <int MINB, bool FP64, bool EDGES, bool STAGE = false>
+template <int MINB, bool FP64, bool EDGES, bool STAGE = false, bool SMALL = false>
 cudaError_t init_engine()
 {
-  return cudaFuncSetAttribute(k_engine<MINB, FP64, EDGES, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_engine<MINB, FP64, EDGES, STAGE, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)engine_smem<STAGE>());
 }
 
@@ -1655,7 +1671,15 @@ cudaError_t dispatch_engine(const KWorldDev* W, EngineArgs A, const Scratch& S, 
       (err = cudaEventRecordWithFlags(S.main_pass_ev[0], s, cudaEventRecordExternal)) != cudaSuccess)
     return err;
   if (A.inline64) return per_sm == 3 ? launch_engine<3, true>(W, A, blocks, s) : launch_engine<2, true>(W, A, blocks, s);
-  switch (per_sm) {
+  const int sms = per_sm > 0 && blocks / per_sm > 0 ? blocks / per_sm : 1;
+  // few edges: the SMALL kernel, with the registers of 2 blocks per SM whatever
+  // the option (there are warps to spare); 1,500 edges are no faster with it
+  const bool small = A.mode == MODE_EDGES && A.stage_nodes == 0 && A.E <= kSmallEdges;
+  switch (small ? 0 : per_sm) {
+    case 0:
+      k_engine<2, false, true, false, true><<<2 * sms, kWarps * 32, engine_smem<false>(), s>>>(W, A);
+      err = cudaGetLastError();
+      break;
     case 3: err = launch_engine<3, false>(W, A, blocks, s); break;
     case 4: err = launch_engine<4, false>(W, A, blocks, s); break;
     default:
@@ -1666,7 +1690,6 @@ cudaError_t dispatch_engine(const KWorldDev* W, EngineArgs A, const Scratch& S, 
   if (S.main_pass_ev[1] != nullptr &&
       (err = cudaEventRecordWithFlags(S.main_pass_ev[1], s, cudaEventRecordExternal)) != cudaSuccess)
     return err;
-  const int sms = per_sm > 0 && blocks / per_sm > 0 ? blocks / per_sm : 1;
   k_band<<<sms, kWarps * 32, 0, s>>>(W, A);
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
   A.head = S.counters + 2;
@@ -1693,6 +1716,7 @@ cudaError_t engine_init()
   if (e == cudaSuccess) e = init_engine<3, true, false>();
   if (e == cudaSuccess) e = init_engine<2, false, true, true>();
   if (e == cudaSuccess) e = init_engine<2, false, false, true>();
+  if (e == cudaSuccess) e = init_engine<2, false, true, false, true>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_self_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(WarpSmem) * kWarps + sizeof(BlockShare)));
