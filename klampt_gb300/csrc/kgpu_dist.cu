@@ -36,6 +36,7 @@
 //     (prismatic), with u = dd/dp at the link feature point p, accumulated as
 //     per-link force/moment sums and pulled back through the chain once per
 //     configuration (the adjoint of FK), on FP32 transforms.
+#include <cstddef>
 #include <cfloat>
 #include <climits>
 
@@ -52,19 +53,23 @@ constexpr int kDPairs = 128;   // gathered (link, object) candidates
 constexpr double kSoftK = 30.0;  // pairs beyond m + 30 tau weigh < e^-30 of the leading term
 
 struct __align__(16) DistSmem {
+  // what a pair's evaluation needs ...
   PairSmem P;
-  uint32_t gstack[kDGStack];
-  int pobj[kDPairs];
-  int plink[kDPairs];
-  float plb[kDPairs];
   float T[kMaxLinks][12];
   float delta[kMaxLinks];
-  float F[kMaxLinks][3], M[kMaxLinks][3];
   double q64[kMaxLinks];
   const float* item_qa;
   const float* item_qb;
   int item_k, item_n;
+  // ... and what gathering the pairs and the gradient need besides: kernels
+  // that only evaluate pairs leave it out (kEvalSmem), and the L1 gains it
+  __align__(16) uint32_t gstack[kDGStack];
+  int pobj[kDPairs];
+  int plink[kDPairs];
+  float plb[kDPairs];
+  float F[kMaxLinks][3], M[kMaxLinks][3];
 };
+constexpr size_t kEvalSmem = offsetof(DistSmem, gstack);
 
 struct DistArgs {
   int mode;            // 0 min distance, 1 soft-min pass 1 (minimum), 2 soft-min pass 2
@@ -372,10 +377,14 @@ __device__ __noinline__ void eval_pair(DistSmem& S, const KWorldDev* __restrict_
     const double d = kx_sqrt(S.P.b2);
     out.found = d < bound;
     out.d = d;
+    // (the three divisions on three lanes: one FP64 sequence instead of three)
+    const int c = lane < 3 ? lane : 0;
+    const float dir = (float)((S.P.bcp[c] - S.P.bcq[c]) / d);
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       out.cp[i] = S.P.bcp[i];
       out.cq[i] = S.P.bcq[i];
-      out.dir[i] = (float)((S.P.bcp[i] - S.P.bcq[i]) / d);
+      out.dir[i] = __shfl_sync(0xffffffffu, dir, i);
     }
     return;
   }
@@ -443,7 +452,7 @@ __device__ int gather_objects(DistSmem& S, const KWorldDev* __restrict__ W, cons
       const float gy = fmaxf(0.f, fabsf(A.c.y - nb.a.y) - nb.b.y);
       const float gz = fmaxf(0.f, fabsf(A.c.z - nb.a.z) - nb.b.z);
       lbv = fmaxf(box_dist32(A, make_float3(nb.a.x, nb.a.y, nb.a.z), make_float3(nb.b.x, nb.b.y, nb.b.z)),
-                  sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU) - rad) -
+                  root_below32(gx * gx + gy * gy + gz * gz) - rad) -
             slack;
       if (lbv <= bound) {
         const int o = W->node_obj[node];
@@ -957,7 +966,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_soft_eval(const KWorldDev* __re
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  DistSmem& S = reinterpret_cast<DistSmem*>(smem_raw)[warp];
+  DistSmem& S = *reinterpret_cast<DistSmem*>(smem_raw + kEvalSmem * warp);
   const KRobotDev& R = W->robots[A.robot];
   const unsigned total = min(*A.count, (unsigned)A.cap);
   DCnt cnt;
@@ -1532,11 +1541,11 @@ cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, con
       if (pass == 1) {
         k_soft_bound<<<some, kDW * 32, smem, s>>>(Wd, A);
         k_soft_gather<1><<<some, kDW * 32, smem, s>>>(Wd, A);
-        k_soft_eval<1><<<2 * num_sms, kDW * 32, smem, s>>>(Wd, A);
+        k_soft_eval<1><<<2 * num_sms, kDW * 32, kEvalSmem * kDW, s>>>(Wd, A);
         k_dist<1><<<some, kDW * 32, smem, s>>>(Wd, D);
       } else {
         k_soft_gather<2><<<some, kDW * 32, smem, s>>>(Wd, A);
-        k_soft_eval<2><<<2 * num_sms, kDW * 32, smem, s>>>(Wd, A);
+        k_soft_eval<2><<<2 * num_sms, kDW * 32, kEvalSmem * kDW, s>>>(Wd, A);
         k_dist<2><<<some, kDW * 32, smem, s>>>(Wd, D);
         k_soft_reduce<<<warps, kDW * 32, smem, s>>>(Wd, A);
       }

@@ -13,12 +13,23 @@
 
 namespace kgpu {
 
+// Square root for lower bounds: within 2^-22 of the root (one instruction, where
+// the rounded one is a dozen and a call; the bounds' code is what the distance
+// kernels fetch most).  root_below32 is not above the true root.
+__device__ __forceinline__ float root_approx32(float x)
+{
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float root_below32(float x) { return root_approx32(x) * (1.f - 16.f * kU); }
+
 __device__ __forceinline__ float box_dist32(const Box32& A, float3 c, float3 h)
 {
   float gx = fmaxf(0.f, fabsf(A.c.x - c.x) - A.h.x - h.x);
   float gy = fmaxf(0.f, fabsf(A.c.y - c.y) - A.h.y - h.y);
   float gz = fmaxf(0.f, fabsf(A.c.z - c.z) - A.h.z - h.z);
-  return sqrtf(gx * gx + gy * gy + gz * gz);
+  return root_below32(gx * gx + gy * gy + gz * gz);
 }
 
 __device__ __forceinline__ float warp_min(float v)
@@ -194,13 +205,18 @@ __device__ __forceinline__ float feature_thr2(const float3* P, const float3* Q, 
   return thr * thr * (1.f + 1e-5f) + 2e-5f * span * span;  // (FLT_MAX bounds overflow to inf: every feature kept)
 }
 
-// lexicographic (d2, a, b) minimum across the warp; result in every lane
-__device__ __forceinline__ void warp_lexmin(double& d2, int& a, int& b, int& src, int lane)
+// Non-negative doubles compare like their bits (integer instructions: an FP64
+// comparison occupies the SM for 19 cycles)
+__device__ __forceinline__ unsigned long long double_bits(double d) { return (unsigned long long)__double_as_longlong(d); }
+
+// lexicographic (d2, a, b) minimum across the warp, d2 as double_bits; result
+// in every lane
+__device__ __forceinline__ void warp_lexmin(unsigned long long& d2, int& a, int& b, int& src, int lane)
 {
   src = lane;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const double od = __shfl_xor_sync(0xffffffffu, d2, o);
+    const unsigned long long od = __shfl_xor_sync(0xffffffffu, d2, o);
     const int oa = __shfl_xor_sync(0xffffffffu, a, o);
     const int ob = __shfl_xor_sync(0xffffffffu, b, o);
     const int os = __shfl_xor_sync(0xffffffffu, src, o);
@@ -212,8 +228,8 @@ __device__ __forceinline__ void warp_lexmin(double& d2, int& a, int& b, int& src
 // Lower bound on the distance of two triangles from the separating direction
 // through their centroids (projections onto a unit vector are 1-Lipschitz);
 // nearly tight for facing triangles, which the box bound is not.  The FP32
-// rounding of the centroids, the normalisation and the projections is
-// covered by the (1 - 8u) factor and the 16 u span term.
+// rounding of the centroids, the normalisation (rsqrtf: 2 ulp) and the
+// projections is covered by the (1 - 16u) factor and the 16 u span term.
 __device__ __forceinline__ float tri_axis_lb32(const float3* P, const float3* Q, float span)
 {
   const float k3 = 1.f / 3.f;
@@ -222,9 +238,9 @@ __device__ __forceinline__ float tri_axis_lb32(const float3* P, const float3* Q,
   const float3 cQ = make_float3((Q[0].x + Q[1].x + Q[2].x) * k3, (Q[0].y + Q[1].y + Q[2].y) * k3,
                                 (Q[0].z + Q[1].z + Q[2].z) * k3);
   float3 u = sub3(cQ, cP);
-  const float nn = sqrtf(dot3(u, u));
-  if (!(nn > 1e-20f)) return 0.f;
-  const float inv = 1.f / nn;
+  const float nn = dot3(u, u);
+  if (!(nn > 1e-30f)) return 0.f;
+  const float inv = rsqrtf(nn);
   u = make_float3(u.x * inv, u.y * inv, u.z * inv);
   float pm = -FLT_MAX, qm = FLT_MAX;
 #pragma unroll
@@ -232,7 +248,7 @@ __device__ __forceinline__ float tri_axis_lb32(const float3* P, const float3* Q,
     pm = fmaxf(pm, dot3(sub3(P[k], cP), u));
     qm = fminf(qm, dot3(sub3(Q[k], cP), u));
   }
-  return (qm - pm) * (1.f - 8.f * kU) - 16.f * kU * span;
+  return (qm - pm) * (1.f - 16.f * kU) - 16.f * kU * span;
 }
 
 }  // namespace kgpu

@@ -26,7 +26,7 @@
 
 namespace kgpu {
 
-constexpr int kPStack = 512;  // node-pair stack entries per warp
+constexpr int kPStack = 384;  // node-pair stack entries per warp (512 takes L1 from the rest, 256 narrows wide fronts)
 constexpr int kPJobs = 64;    // leaf pairs
 constexpr int kPFull = 64;    // triangle pairs for the full FP32 distance
 constexpr int kPCand = 64;    // FP64 candidates
@@ -102,7 +102,7 @@ __device__ __forceinline__ float tri_box_lb32(const float3* P, const float3* Q)
   const float gx = fmaxf(0.f, fmaxf(ql.x - ph.x, pl.x - qh.x));
   const float gy = fmaxf(0.f, fmaxf(ql.y - ph.y, pl.y - qh.y));
   const float gz = fmaxf(0.f, fmaxf(ql.z - ph.z, pl.z - qh.z));
-  return sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU);
+  return root_below32(gx * gx + gy * gy + gz * gz);
 }
 
 // FP64 finalisation of the candidates still within the band of m32, merged
@@ -161,13 +161,14 @@ __device__ __noinline__ int pair_flush(PairSmem& S, const MeshView& A, const Mes
       ++done;
     }
     int src;
-    double m2 = d2;
+    unsigned long long m2 = double_bits(d2);
     int ma = oa, mb = ob;
     warp_lexmin(m2, ma, mb, src, lane);
     // below the acceptance bound, or equal to the best with smaller triangles
-    const bool better = S.have ? (m2 < S.b2 || (m2 == S.b2 && (ma < S.bA || (ma == S.bA && mb < S.bB)))) : m2 < S.b2;
+    const unsigned long long b2 = double_bits(S.b2);
+    const bool better = m2 < b2 || (S.have && m2 == b2 && (ma < S.bA || (ma == S.bA && mb < S.bB)));
     __syncwarp();
-    if (m2 < DBL_MAX && better && lane == src) {
+    if (m2 < double_bits(DBL_MAX) && better && lane == src) {
       S.b2 = d2;
       S.bA = oa;
       S.bB = ob;
@@ -206,7 +207,7 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
         d32 = 0.f;
         if (CERT) certain = tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd);
       } else {
-        d32 = sqrtf(tri_dist2_32(P[0], P[1], P[2], Q[0], Q[1], Q[2]));
+        d32 = root_approx32(tri_dist2_32(P[0], P[1], P[2], Q[0], Q[1], Q[2]));
       }
     }
   }
@@ -255,10 +256,9 @@ __device__ __forceinline__ float node_lb32(const MeshView& A, const MeshView& B,
     const float gx = fmaxf(0.f, fabsf(d.x) - BB.h.x);
     const float gy = fmaxf(0.f, fabsf(d.y) - BB.h.y);
     const float gz = fmaxf(0.f, fabsf(d.z) - BB.h.z);
-    lb = fmaxf(lb, sqrtf(gx * gx + gy * gy + gz * gz) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA));
+    lb = fmaxf(lb, root_below32(gx * gx + gy * gy + gz * gz) - __ldg(A.node_r + nodeA));
   } else {
-    lb = fmaxf(lb, sqrtf(d.x * d.x + d.y * d.y + d.z * d.z) * (1.f - 4.f * kU) - __ldg(A.node_r + nodeA) -
-                       __ldg(B.node_r + nodeB));
+    lb = fmaxf(lb, root_below32(n2) - __ldg(A.node_r + nodeA) - __ldg(B.node_r + nodeB));
   }
   // separation along the line of centres: both boxes projected onto it
   // (columns of T give the rotated box's half widths along d).  Boxes small
@@ -314,7 +314,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
         ready();
         cnt.fp64 += pair_flush<IDB>(S, A, B, TA, TB, TA64, TB64, lane, ncand, m32, dd);
         ncand = 0;
-        if (S.have) m32 = fminf(m32, (float)sqrt(S.b2) * (1.f + 1e-6f));
+        if (S.have) m32 = fminf(m32, sqrtf((float)S.b2) * (1.f + 2e-6f));
       }
       const int r = pair_full<IDB, CERT>(S, A, B, TA, TB, lane, nfull, ncand, dd, m32);
       if (CERT && r < 0) {
@@ -332,16 +332,19 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
       bool go = false;
       float lb = 0.f;
       int tA = 0, tB = 0;
+      // the leaf pair of each lane: the number of leaf pairs that start at or
+      // before its position, from a bit mask of the starts in this window
+      const uint32_t o0 = lane < njobs ? S.jobOff[lane] : ~0u, o1 = lane + 32 < njobs ? S.jobOff[lane + 32] : ~0u;
+      const uint32_t starts = __reduce_or_sync(0xffffffffu, (o0 - jpos < 32u ? 1u << (o0 - jpos) : 0u) |
+                                                                (o1 - jpos < 32u ? 1u << (o1 - jpos) : 0u));
+      const int before = __popc(__ballot_sync(0xffffffffu, o0 < jpos)) + __popc(__ballot_sync(0xffffffffu, o1 < jpos));
       if (p < jtotal) {
-        int lo = 0, hi = njobs - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (S.jobOff[mid] <= p) lo = mid; else hi = mid - 1;
-        }
-        const uint32_t r = p - S.jobOff[lo];
-        const uint32_t cb = (S.jobB[lo] >> 28) + 1;
-        tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
-        tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
+        const int j = before + __popc(starts & (lt | (1u << lane))) - 1;
+        const uint32_t r = p - S.jobOff[j], cb = (S.jobB[j] >> 28) + 1;
+        // r / cb for r < 16, cb <= 4
+        const uint32_t ra = (r * (cb == 3 ? 21846u : 65536u >> (cb >> 1))) >> 16;
+        tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
+        tB = (int)((S.jobB[j] & 0x0fffffffu) + r - ra * cb);
         float3 P[3], Q[3];
         place32<false>(A, TA, tA, P);
         place32<IDB>(B, TB, tB, Q);
@@ -443,7 +446,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
   if (ncand > 0) {
     ready();
     cnt.fp64 += pair_flush<IDB>(S, A, B, TA, TB, TA64, TB64, lane, ncand, m32, dd);
-    if (S.have) m32 = fminf(m32, (float)sqrt(S.b2) * (1.f + 1e-6f));
+    if (S.have) m32 = fminf(m32, sqrtf((float)S.b2) * (1.f + 2e-6f));
   }
   return 0;
 }
