@@ -14,7 +14,7 @@
 //   * One warp processes one work item (a configuration or an edge step) at
 //     a time and pulls items from a device work queue (persistent grid sized
 //     to the SM count).  An edge item is a chunk of consecutive steps
-//     (`chunk`, default 4) checked in order; chunks are ordered round-major
+//     (`chunk`, default 16) checked in order; chunks are ordered round-major
 //     across edges, so every edge's early steps run first and a step beyond
 //     an edge's first collision is skipped.
 //   * FK: lane i owns link i (warp_fk32); transforms go to shared memory.
@@ -239,19 +239,15 @@ __device__ __noinline__ unsigned run_jobs(WarpSmem& S, const KWorldDev* __restri
   const uint32_t total = carry;
   const float4* __restrict__ ltri = W->ltri32;
   const float4* __restrict__ etri = W->etri32;
+  int jb = 0;
 #pragma unroll 1
   for (uint32_t base = 0; base < total; base += 32) {
     uint32_t p = base + lane;
+    const uint32_t starts = window_starts(S.jobOff, jb, njobs, base, lane);
     bool band = false, certain = false, mine = false;
     int la = 0, tgt = 0, tA = 0, tB = 0, step = 0;
     if (p < total) {
-      // job holding p: largest j with jobOff[j] <= p
-      int lo = 0, hi = njobs - 1;
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (S.jobOff[mid] <= p) lo = mid; else hi = mid - 1;
-      }
-      const int j = lo;
+      const int j = jb + __popc(starts & ((2u << lane) - 1u)) - 1;
       const uint32_t jm = S.jobM[j];
       la = jm & 0xff;
       tgt = (jm >> 8) & 0xff;
@@ -260,8 +256,9 @@ __device__ __noinline__ unsigned run_jobs(WarpSmem& S, const KWorldDev* __restri
       if (mine) {
         const uint32_t r = p - S.jobOff[j];
         const uint32_t cb = ((jm >> 16) & 3u) + 1;
-        tA = (int)(S.jobA[j] & 0x0fffffffu) + (int)(r / cb);
-        tB = (int)S.jobB[j] + (int)(r % cb);
+        const uint32_t ra = leaf_quotient(r, cb);
+        tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
+        tB = (int)(S.jobB[j] + r - ra * cb);
         float3 P[3], Q[3];
         const bool self = tgt < 32;
         float TA[12], TB[12];
@@ -284,6 +281,7 @@ __device__ __noinline__ unsigned run_jobs(WarpSmem& S, const KWorldDev* __restri
         cnt.tri_pairs++;
       }
     }
+    jb += __popc(starts);
     if (__any_sync(0xffffffffu, certain)) {
       cnt.cert++;
       const unsigned hm = __reduce_or_sync(0xffffffffu, certain ? 1u << step : 0u);

@@ -223,6 +223,25 @@ __device__ __forceinline__ float rot_gram_err32(const float* P)
   return g + 8.f * kU;
 }
 
+// Leaf pairs expand to one triangle pair per lane, window of 32 after window.
+// The leaf pairs that start in the window at `base`, as a bit mask: at most 32,
+// since each has a pair; `before` start in earlier windows, so lane l is in the
+// one before + popc(mask up to bit l) - 1.  (A binary search over the offsets
+// and an integer division instead of leaf_quotient cost 262,144 configurations
+// 4.77 ms, now 4.56, 500 feasibility checks 246 us, now 228, 16,384 edges 1,623
+// us, now 1,593: the divergent loop's instructions are fetched for every window.)
+__device__ __forceinline__ uint32_t window_starts(const uint32_t* off, int before, int n, uint32_t base, int lane)
+{
+  const uint32_t at = before + lane < n ? off[before + lane] - base : 32u;
+  return __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+}
+
+// r / c for r < 16 and 1 <= c <= 4 (triangles of a leaf)
+__device__ __forceinline__ uint32_t leaf_quotient(uint32_t r, uint32_t c)
+{
+  return (r * (c == 3 ? 21846u : 65536u >> (c >> 1))) >> 16;
+}
+
 struct Box32 {
   float3 c, h;
 };
@@ -406,9 +425,8 @@ __device__ __forceinline__ void chain64(const KRobotDev& R, const double* q64, i
 // order exactly as the oracle does (T[i] = T[parent] * L_i), one matrix entry
 // per lane, so the result is bit-identical to the sequential chain.  (An FP64
 // instruction costs the SM 19 cycles whatever its active lanes: a product is 6
-// instead of 66 of them. 
-// 32,768 terrain clearances 27.8 -> 26.1 ms, 8,192 humanoid self distances
-// 16.2 -> 15.4 ms.)
+// instead of 66 of them.  Measured: 32,768 terrain clearances 27.8 -> 26.1 ms, 8,192
+// humanoid self distances 16.2 -> 15.4 ms.)
 static __device__ __noinline__ void warp_fk64(const KRobotDev& R, const double* q64, double (*T64)[12],
                                               int lane)
 {

@@ -20,7 +20,8 @@
 //   soft-min      = m - tau log sum exp(-(d - m)/tau) over the trajectory's
 //                   pairs with d < m + K tau (K = 30), m the trajectory minimum.
 //
-// GPU method, one warp per configuration (waypoint):
+// GPU method, one warp per configuration (the soft-min: one warp per pair, see
+// below):
 //   * FP32 FK with per-link error bounds (warp_fk32);
 //   * candidate (link, object) pairs from the object-aware environment tree by
 //     box lower bounds, evaluated nearest first; for the minimum, the bound
@@ -63,6 +64,7 @@ struct __align__(16) DistSmem {
   int item_k, item_n;
   // ... and what gathering the pairs and the gradient need besides: kernels
   // that only evaluate pairs leave it out (kEvalSmem), and the L1 gains it
+  // (soft-min over 6,400 waypoints: 3%)
   __align__(16) uint32_t gstack[kDGStack];
   int pobj[kDPairs];
   int plink[kDPairs];
@@ -187,7 +189,8 @@ __device__ __forceinline__ float depth_band(const KNode& ob, float dd)
 // cycles; the pair's own evaluation (the search for a certified contact, then
 // its deepest vertex in FP64) takes a few hundred thousand.  Among boxes most
 // pairs a configuration still has to look at after its first contact are
-// shallower contacts: 32,768 terrain clearances 38.9 -> 27.4 ms with this test.
+// shallower contacts: 32,768 terrain clearances 38.9 -> 27.4 ms with this test
+// (20.7 with the later work on the pair traversal).
 __device__ __noinline__ bool may_be_deeper(const DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                            int lane, int l, int o, float need)
 {
@@ -763,8 +766,8 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
 // takes pairs from it: one trajectory of 32 waypoints has a few thousand pairs
 // within 30 tau of its minimum, and one waypoint's are up to a few hundred, so
 // a warp per waypoint leaves the GPU idle or waiting for the last ones (one
-// trajectory 20-30 -> 1.7 ms, 200 trajectories 98.5 -> 54 ms).  Per chunk of
-// waypoints:
+// trajectory 33-72 -> 1.7 ms, 200 trajectories 98.5 -> 54 ms; 1.5 and 40 ms with
+// the later work on the pair traversal).  Per chunk of waypoints:
 //   k_soft_fk       FP32 and FP64 forward kinematics, kept for the chunk;
 //   k_soft_bound    an upper bound of each trajectory's minimum, from the
 //                   pairs nearest by their boxes at each waypoint;
@@ -1252,7 +1255,8 @@ __device__ __noinline__ void self_pairs(SelfDistSmem& S, const KWorldDev* __rest
 // (i, j) order evaluated most of a humanoid's 435.  The result is the
 // lexicographic minimum (distance, pair), whatever the order.  Blocks of two
 // warps, so that a costly configuration holds up one other at most.  8,192
-// humanoid configurations: 27.5 -> 5.96 ms (15.4 ms before this order).
+// humanoid configurations: 15.4 -> 5.96 ms by this order (5.15 ms with the
+// later work on the pair traversal).
 __global__ void __launch_bounds__(kSW * 32, 16 / kSW) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];

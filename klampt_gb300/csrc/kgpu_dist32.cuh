@@ -15,7 +15,8 @@ namespace kgpu {
 
 // Square root for lower bounds: within 2^-22 of the root (one instruction, where
 // the rounded one is a dozen and a call; the bounds' code is what the distance
-// kernels fetch most).  root_below32 is not above the true root.
+// kernels fetch most: 7-13% of their time).  root_below32 is not above the true
+// root.
 __device__ __forceinline__ float root_approx32(float x)
 {
   float r;
@@ -137,13 +138,13 @@ static __device__ __noinline__ float tri_dist2_32(float3 P0, float3 P1, float3 P
 // ---- which features the canonical FP64 distance still has to look at --------
 // kx_tri_tri_dist2 is the minimum over 15 features (9 edge-edge, 3 vertices of
 // P against Q, 3 of Q against P; bit 3 i + j, 9 + k, 12 + k), taken in that
-// order with strict comparisons (tri_dist2_masked64).  An FP64 operation occupies the SM for 19
-// cycles per warp whatever the number of active lanes, and all 15 features
+// order with strict comparisons (tri_dist2_masked64).  An FP64 operation
+// occupies the SM for 19 cycles per warp whatever the number of active lanes, and all 15 features
 // plus the 17 overlap axes are ~2,300 of them; in FP32 the features are a few
 // hundred full-rate instructions.  Measured (before -> after): 8,192 humanoid
 // self distances 28.4 -> 20.0 ms, soft-min over 6,400 waypoints 190.5 -> 140.1
-// ms, 32,768 terrain clearances 47.9 -> 43.7 ms.  The mask keeps the features whose FP32
-// squared distance is at most thr2 (the caller's upper bound on the pair's
+// ms, 32,768 terrain clearances 47.9 -> 43.7 ms.  The mask keeps the features
+// whose FP32 squared distance is at most thr2 (the caller's upper bound on the pair's
 // minimum with its bands); the dropped ones cannot be the minimum.
 //
 // An FP32 feature value exceeds the feature's exact one by the placement and

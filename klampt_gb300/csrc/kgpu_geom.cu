@@ -264,20 +264,18 @@ __global__ void __launch_bounds__(kGW * 32) k_geom_collide(const GeomDev GA, con
         }
         __syncwarp();
         const uint32_t total = carry;
+        int jb = 0;
 #pragma unroll 1
         for (uint32_t base = 0; base < total && !hit; base += 32) {
           const uint32_t p = base + lane;
+          const uint32_t starts = window_starts(S.jobOff, jb, njobs, base, lane);
           bool h = false;
           if (p < total) {
-            int lo = 0, hi = njobs - 1;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (S.jobOff[mid] <= p) lo = mid; else hi = mid - 1;
-            }
-            const uint32_t r = p - S.jobOff[lo];
-            const uint32_t cb = (S.jobB[lo] >> 28) + 1;
-            const int tA = (int)(S.jobA[lo] & 0x0fffffffu) + (int)(r / cb);
-            const int tB = (int)(S.jobB[lo] & 0x0fffffffu) + (int)(r % cb);
+            const int j = jb + __popc(starts & ((2u << lane) - 1u)) - 1;
+            const uint32_t r = p - S.jobOff[j];
+            const uint32_t cb = (S.jobB[j] >> 28) + 1, ra = leaf_quotient(r, cb);
+            const int tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
+            const int tB = (int)((S.jobB[j] & 0x0fffffffu) + r - ra * cb);
             float3 P[3], Q[3];
             tri_world32(GA, TA, tA, P);
             tri_world32(GB, TB, tB, Q);
@@ -299,6 +297,7 @@ __global__ void __launch_bounds__(kGW * 32) k_geom_collide(const GeomDev GA, con
             }
           }
           hit = __any_sync(0xffffffffu, h);
+          jb += __popc(starts);
         }
         njobs = 0;
         continue;

@@ -10,8 +10,9 @@
 // become candidates, finalised in FP64 with a lexicographic reduction
 // (squared distance, triangle of A, triangle of B).
 //
-// What bounds it: instruction issue on dependent FP32 chains and the FP64
-// pipe.  A triangle pair's separation test and distance are ~1,600
+// What bounds it: fetching its instructions (the top stall, 30-40% of the
+// samples; half the warps keep 91% of the speed) and the FP64 pipe (25-38% of
+// the time).  A triangle pair's separation test and distance are ~1,600
 // instructions, and of the pairs whose bounds are computed 2-3% need them, so
 // running them where they are found costs 15 warp-wide evaluations a mesh
 // pair with 4-5 lanes active; collected they are 2-3 full ones.  Measured
@@ -19,14 +20,17 @@
 // the node bound along the line of centres: 16,384 cylinder-icosphere
 // distances 8.3 -> 4.0 ms, soft-min over 6,400 waypoints 140 -> 105 ms, 8,192
 // humanoid self distances 20.0 -> 17.9 ms, 32,768 terrain clearances 43.7 ->
-// 38.9 ms.
+// 38.9 ms.  With one-instruction roots in the bounds, leaf-pair positions from
+// a bit mask instead of a binary search and a division, and minima compared as
+// integers, the same four went from 3.9, 45.2, 5.75 and 24.7 ms to 3.5, 39.2,
+// 5.15 and 20.7 ms (mostly by the roots).
 #pragma once
 
 #include "kgpu_dist32.cuh"
 
 namespace kgpu {
 
-constexpr int kPStack = 384;  // node-pair stack entries per warp (512 takes L1 from the rest, 256 narrows wide fronts)
+constexpr int kPStack = 384;  // node-pair stack entries per warp (512: soft-min +2.5%, L1; 256: terrain +20%, narrowed fronts)
 constexpr int kPJobs = 64;    // leaf pairs
 constexpr int kPFull = 64;    // triangle pairs for the full FP32 distance
 constexpr int kPCand = 64;    // FP64 candidates
@@ -302,6 +306,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
   __syncwarp();
   int top = 1, njobs = 0, nfull = 0, ncand = 0;
   uint32_t jpos = 0, jtotal = 0;  // expansion of the leaf pairs in progress
+  int jbefore = 0;                // leaf pairs that start before jpos
   // collected pairs that may touch (lower bound <= 0) are tested at once: a
   // contact certified early ends the search
   bool touch = false;
@@ -332,17 +337,10 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
       bool go = false;
       float lb = 0.f;
       int tA = 0, tB = 0;
-      // the leaf pair of each lane: the number of leaf pairs that start at or
-      // before its position, from a bit mask of the starts in this window
-      const uint32_t o0 = lane < njobs ? S.jobOff[lane] : ~0u, o1 = lane + 32 < njobs ? S.jobOff[lane + 32] : ~0u;
-      const uint32_t starts = __reduce_or_sync(0xffffffffu, (o0 - jpos < 32u ? 1u << (o0 - jpos) : 0u) |
-                                                                (o1 - jpos < 32u ? 1u << (o1 - jpos) : 0u));
-      const int before = __popc(__ballot_sync(0xffffffffu, o0 < jpos)) + __popc(__ballot_sync(0xffffffffu, o1 < jpos));
+      const uint32_t starts = window_starts(S.jobOff, jbefore, njobs, jpos, lane);
       if (p < jtotal) {
-        const int j = before + __popc(starts & (lt | (1u << lane))) - 1;
-        const uint32_t r = p - S.jobOff[j], cb = (S.jobB[j] >> 28) + 1;
-        // r / cb for r < 16, cb <= 4
-        const uint32_t ra = (r * (cb == 3 ? 21846u : 65536u >> (cb >> 1))) >> 16;
+        const int j = jbefore + __popc(starts & (lt | (1u << lane))) - 1;
+        const uint32_t r = p - S.jobOff[j], cb = (S.jobB[j] >> 28) + 1, ra = leaf_quotient(r, cb);
         tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
         tB = (int)((S.jobB[j] & 0x0fffffffu) + r - ra * cb);
         float3 P[3], Q[3];
@@ -366,6 +364,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
       nfull += __popc(mg);
       if (CERT) touch = __any_sync(0xffffffffu, go && lb <= 0.f);
       jpos += 32;
+      jbefore += __popc(starts);
       if (jpos >= jtotal) {
         jpos = jtotal = 0;
         njobs = 0;
@@ -391,6 +390,7 @@ __device__ __forceinline__ int pair_distance(PairSmem& S, const MeshView& A, con
       __syncwarp();
       jtotal = carry;
       jpos = 0;
+      jbefore = 0;
       continue;
     }
     // ---- node pairs.  A batch of n pops grows the stack by at most n; near
