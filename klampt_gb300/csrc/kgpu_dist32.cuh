@@ -13,18 +13,6 @@
 
 namespace kgpu {
 
-// Square root for lower bounds: within 2^-22 of the root (one instruction, where
-// the rounded one is a dozen and a call; the bounds' code is what the distance
-// kernels fetch most: 7-13% of their time).  root_below32 is not above the true
-// root.
-__device__ __forceinline__ float root_approx32(float x)
-{
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float root_below32(float x) { return root_approx32(x) * (1.f - 16.f * kU); }
-
 __device__ __forceinline__ float box_dist32(const Box32& A, float3 c, float3 h)
 {
   float gx = fmaxf(0.f, fabsf(A.c.x - c.x) - A.h.x - h.x);
