@@ -224,6 +224,27 @@ __global__ void __launch_bounds__(kGW * 32) k_geom_distance(const GeomDev GA, co
   }
 }
 
+// Whether two triangles are within the threshold, as far as FP32 can say:
+// kWithinYes, kWithinApart alone (no), or the features that the FP64 decision
+// has to look at, with kWithinApart where the overlap test is settled.  The
+// FP32 distance is that of two points of the triangles, so with its band it
+// bounds the distance from above, whatever the triangles' shape; a feature
+// beyond the threshold (mlo, m32: it, rounded down and up) and its bands cannot
+// be a minimum within it.  (All 15 features in FP64 for every pair that the
+// separating axes leave: 2,864 queries 2,294 us at a 5 cm tolerance, now 829;
+// 571 of finer meshes 2,856, now 1,166.)
+constexpr unsigned kWithinYes = 1u << 16, kWithinApart = 1u << 17;
+
+static __device__ __noinline__ unsigned within32(float3 P0, float3 P1, float3 P2, float3 Q0, float3 Q1, float3 Q2,
+                                                 float mlo, float m32, float dd)
+{
+  const float3 P[3] = {P0, P1, P2}, Q[3] = {Q0, Q1, Q2};
+  const float e = dd + 128.f * kU * tri_span(P, Q) + 1e-8f;
+  if ((root_approx32(tri_dist2_32(P0, P1, P2, Q0, Q1, Q2)) + e) * (1.f + 1e-5f) <= mlo) return kWithinYes;
+  if (!tri_separated32(P, Q, dd, 0.f)) return kFeatAll;
+  return kWithinApart | tri_feature_mask32(P0, P1, P2, Q0, Q1, Q2, feature_thr2(P, Q, m32, dd));
+}
+
 __global__ void __launch_bounds__(kGW * 32) k_geom_collide(const GeomDev GA, const GeomDev GB, const GeomArgs A)
 {
   __shared__ GeomSmem smem[kGW];
@@ -269,35 +290,45 @@ __global__ void __launch_bounds__(kGW * 32) k_geom_collide(const GeomDev GA, con
         for (uint32_t base = 0; base < total && !hit; base += 32) {
           const uint32_t p = base + lane;
           const uint32_t starts = window_starts(S.jobOff, jb, njobs, base, lane);
-          bool h = false;
+          bool certain = false, band = false;
+          int tA = 0, tB = 0;
+          unsigned look = kFeatAll;
           if (p < total) {
             const int j = jb + __popc(starts & ((2u << lane) - 1u)) - 1;
             const uint32_t r = p - S.jobOff[j];
             const uint32_t cb = (S.jobB[j] >> 28) + 1, ra = leaf_quotient(r, cb);
-            const int tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
-            const int tB = (int)((S.jobB[j] & 0x0fffffffu) + r - ra * cb);
+            tA = (int)((S.jobA[j] & 0x0fffffffu) + ra);
+            tB = (int)((S.jobB[j] & 0x0fffffffu) + r - ra * cb);
             float3 P[3], Q[3];
             tri_world32(GA, TA, tA, P);
             tri_world32(GB, TB, tB, Q);
             if (!tri_separated32(P, Q, dd, m32)) {
-              if (A.m == 0.0 && tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd)) {
-                h = true;
+              if (A.m == 0.0) {
+                certain = tri_certain_hit32(P[0], P[1], P[2], Q[0], Q[1], Q[2], dd);
               } else {
-                // the band: the canonical FP64 decision
-                double P64[9], Q64[9];
-                tri_world64(GA, G.T64[0], tA, P64);
-                tri_world64(GB, G.T64[1], tB, Q64);
-                if (A.m == 0.0) {
-                  h = tri_overlap64(P64, Q64) != 0;
-                } else {
-                  double c1[3], c2[3];
-                  h = tri_dist2_masked64(P64, Q64, kFeatAll, false, c1, c2) <= kx_mul(A.m, A.m);
-                }
+                look = within32(P[0], P[1], P[2], Q[0], Q[1], Q[2], (float)A.m * (1.f - 1e-6f), m32, dd);
+                certain = (look & kWithinYes) != 0;
               }
+              band = !certain && look != kWithinApart;
+            }
+          }
+          jb += __popc(starts);
+          hit = __any_sync(0xffffffffu, certain);
+          if (hit) break;
+          bool h = false;
+          if (band) {
+            // the canonical FP64 decision
+            double P64[9], Q64[9];
+            tri_world64(GA, G.T64[0], tA, P64);
+            tri_world64(GB, G.T64[1], tB, Q64);
+            if (A.m == 0.0) {
+              h = tri_overlap64(P64, Q64) != 0;
+            } else {
+              double c1[3], c2[3];
+              h = tri_dist2_masked64(P64, Q64, look, (look & kWithinApart) != 0, c1, c2) <= kx_mul(A.m, A.m);
             }
           }
           hit = __any_sync(0xffffffffu, h);
-          jb += __popc(starts);
         }
         njobs = 0;
         continue;
