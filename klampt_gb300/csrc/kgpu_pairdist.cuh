@@ -10,9 +10,9 @@
 // become candidates, finalised in FP64 with a lexicographic reduction
 // (squared distance, triangle of A, triangle of B).
 //
-// What bounds it: fetching its instructions (the top stall, 30-40% of the
-// samples; half the warps keep 91% of the speed) and the FP64 pipe (25-38% of
-// the time).  A triangle pair's separation test and distance are ~1,600
+// What bounds it: fetching its instructions (the soft-min's top stall, 41% of
+// the samples; half the warps keep 91% of the speed), load latency, and in the
+// soft-min the FP64 pipe (26% busy).  A triangle pair's separation test and distance are ~1,600
 // instructions, and of the pairs whose bounds are computed 2-3% need them, so
 // running them where they are found costs 15 warp-wide evaluations a mesh
 // pair with 4-5 lanes active; collected they are 2-3 full ones.  Measured
