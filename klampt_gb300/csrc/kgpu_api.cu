@@ -553,7 +553,8 @@ kgpu_status kgpu_env_create_ex(const kgpu_env_desc* d, int32_t flags, kgpu_env* 
     int t = leaf_tris[k];
     for (int v = 0; v < 3; ++v)
       tri32[3 * k + v] = make_float4((float)E->tri64[9 * (size_t)t + 3 * v], (float)E->tri64[9 * (size_t)t + 3 * v + 1],
-                                     (float)E->tri64[9 * (size_t)t + 3 * v + 2], 0.f);
+                                     (float)E->tri64[9 * (size_t)t + 3 * v + 2],
+                                     v == 0 ? flat_mark(&E->tri64[9 * (size_t)t]) : 0.f);
     for (int i = 0; i < 9; ++i) tri64l[9 * k + i] = E->tri64[9 * (size_t)t + i];
     tobj[k] = E->tri_obj[t];
   }
@@ -648,7 +649,8 @@ kgpu_status kgpu_world_create(kgpu_env env, const kgpu_robot* robots, int32_t n,
     for (int l = 0; l < R->nlinks; ++l) {
       append_bvh(R->bvh[l], (int)nodes.size(), (int)(tri32.size() / 3), nodes, node64, &lnode_r);
       for (size_t k = 0; k < R->tri64[l].size(); k += 3)
-        tri32.push_back(make_float4((float)R->tri64[l][k], (float)R->tri64[l][k + 1], (float)R->tri64[l][k + 2], 0.f));
+        tri32.push_back(make_float4((float)R->tri64[l][k], (float)R->tri64[l][k + 1], (float)R->tri64[l][k + 2],
+                                    k % 9 == 0 ? flat_mark(&R->tri64[l][k]) : 0.f));
       tri64.insert(tri64.end(), R->tri64[l].begin(), R->tri64[l].end());
       for (int t : R->bvh[l].order) ltri_orig.push_back(t);
       for (size_t k = 0; k < R->vert64[l].size(); k += 3) {

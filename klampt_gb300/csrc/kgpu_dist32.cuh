@@ -168,7 +168,7 @@ static __device__ __noinline__ unsigned tri_feature_mask32(float3 P0, float3 P1,
     const float L2 = fmaxf(dot3(ab, ab), fmaxf(dot3(ac, ac), dot3(bc, bc)));
     const float n2 = dot3(n, n);
     const bool thin = !(n2 >= 0.01f * L2 * L2);
-    if (!(n2 >= 1e-8f * L2 * L2)) mask |= kFeatFlat;
+    if (!(n2 > 1e-8f * L2 * L2)) mask |= kFeatFlat;  // (a single point too)
 #pragma unroll 1
     for (int k = 0; k < 3; ++k) {
       const float3 p = t ? sel3(k, Q0, Q1, Q2) : sel3(k, P0, P1, P2);

@@ -511,7 +511,8 @@ extern "C" kgpu_status kgpu_geom_create(const kgpu_geom_desc* d, kgpu_geom* out)
       orig.push_back(t);
       for (int v = 0; v < 3; ++v)
         t32.push_back(make_float4((float)tri[9 * (size_t)t + 3 * v], (float)tri[9 * (size_t)t + 3 * v + 1],
-                                  (float)tri[9 * (size_t)t + 3 * v + 2], 0.f));
+                                  (float)tri[9 * (size_t)t + 3 * v + 2],
+                                  v == 0 ? flat_mark(&tri[9 * (size_t)t]) : 0.f));
       for (int i = 0; i < 9; ++i) t64.push_back(tri[9 * (size_t)t + i]);
     }
   }

@@ -82,12 +82,33 @@ struct KRobotDev {
   double link_margin64[kMaxLinks];
 };
 
+// Mark of a triangle without area (1, otherwise 0), kept in the fourth word of
+// its first FP32 vertex.  The canonical overlap test has no normal of such a
+// triangle to separate along and can report a contact of triangles that are
+// apart, which no FP32 distance foresees: the distance kernels leave every
+// reached pair with one to the canonical function.
+inline float flat_mark(const double* t)
+{
+  double e[3][3], l2 = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    double s = 0.0;
+    for (int i = 0; i < 3; ++i) {
+      e[k][i] = t[3 * ((k + 1) % 3) + i] - t[3 * k + i];
+      s += e[k][i] * e[k][i];
+    }
+    l2 = s > l2 ? s : l2;
+  }
+  const double x = e[0][1] * e[1][2] - e[0][2] * e[1][1], y = e[0][2] * e[1][0] - e[0][0] * e[1][2],
+               z = e[0][0] * e[1][1] - e[0][1] * e[1][0];
+  return x * x + y * y + z * z > 2e-8 * l2 * l2 ? 0.f : 1.f;
+}
+
 struct KWorldDev {
   // robots
   const KRobotDev* robots;
   const uint32_t* queries;   // a | tgt << 8 ; tgt < 32: link, tgt >= 32: env group tgt-32
   const KNode* lnodes;
-  const float4* ltri32;      // 3 per tri
+  const float4* ltri32;      // 3 per tri; .w of the first: flat_mark
   const double* ltri64;      // 9 per tri
   const double* lnode64;     // 6 per node (c, h) FP64 (plain kernel)
   const float* lnode_r;      // per link node: radius about its FP32 centre holding its vertices

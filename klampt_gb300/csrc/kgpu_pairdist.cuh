@@ -38,7 +38,7 @@ constexpr int kPCand = 64;    // FP64 candidates
 struct MeshView {
   const KNode* nodes;
   const float* node_r;  // radius per node about its FP32 centre, or null
-  const float4* tri32;  // 3 per triangle, leaf order
+  const float4* tri32;  // 3 per triangle, leaf order; .w of the first: flat_mark
   const double* tri64;  // 9 per triangle
   const int* orig;      // leaf order -> mesh order
 };
@@ -195,7 +195,7 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
 {
   const int n = min(nfull, 32);
   float d32 = FLT_MAX, e = 0.f;
-  bool certain = false;
+  bool certain = false, flat = false;
   int tA = 0, tB = 0;
   if (lane < n) {
     const int k = nfull - 1 - lane;
@@ -206,6 +206,7 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
       place32<false>(A, TA, tA, P);
       place32<IDB>(B, TB, tB, Q);
       e = dd + 128.f * kU * tri_span(P, Q) + 1e-8f;
+      flat = __ldg(&A.tri32[3 * (size_t)tA].w) + __ldg(&B.tri32[3 * (size_t)tB].w) > 0.f;
       // (a positive lower bound, bands included, has them apart already)
       if (!(S.fullL[k] > 0.f) && !tri_separated32(P, Q, dd, 0.f)) {
         d32 = 0.f;
@@ -220,14 +221,15 @@ __device__ __noinline__ int pair_full(PairSmem& S, const MeshView& A, const Mesh
     if (mc) return -1 - __shfl_sync(0xffffffffu, tA, __ffs(mc) - 1);
   }
   m32 = fminf(m32, warp_min(d32 < FLT_MAX ? d32 + e : FLT_MAX));
-  const bool cand = d32 < FLT_MAX && d32 - e <= m32 * (1.f + 2e-5f);
+  // (a triangle without area: a contact for the canonical function, maybe)
+  const bool cand = d32 < FLT_MAX && (flat || d32 - e <= m32 * (1.f + 2e-5f));
   const unsigned mk = __ballot_sync(0xffffffffu, cand);
   if (cand) {
     const int r = ncand + __popc(mk & lanemask_lt());
     S.candA[r] = (uint32_t)tA;
     S.candB[r] = (uint32_t)tB;
-    S.candD[r] = d32 - e;
-    S.candS[r] = d32 > 0.f;
+    S.candD[r] = flat ? 0.f : d32 - e;
+    S.candS[r] = d32 > 0.f && !flat;
   }
   __syncwarp();
   return ncand + __popc(mk);
