@@ -61,44 +61,49 @@ static __device__ float seg_seg2_32(float3 p1, float3 d1, float3 p2, float3 d2)
   return dot3(w, w);
 }
 
+// The callers take the value with its band as an upper bound.  So the foot is
+// a point of the triangle whatever its shape (weights clamped: a sliver's are
+// rounding noise), and it is formed relative to the vertices, never in world
+// coordinates: its rounding then scales with the span, as the band does, not
+// with the distance from the origin (a 0.1 mm triangle at 0.3 m was off by up
+// to 2e-8 beyond that band).
 static __device__ float pt_tri2_32(float3 p, float3 a, float3 b, float3 c)
 {
   const float3 ab = sub3(b, a), ac = sub3(c, a), ap = sub3(p, a);
   const float d1 = dot3(ab, ap), d2 = dot3(ac, ap);
-  float3 q;
-  if (d1 <= 0.f && d2 <= 0.f) { q = a; goto done; }
+  float3 w;  // p - foot
+  if (d1 <= 0.f && d2 <= 0.f) { w = ap; goto done; }
   {
     const float3 bp = sub3(p, b);
     const float d3 = dot3(ab, bp), d4 = dot3(ac, bp);
-    if (d3 >= 0.f && d4 <= d3) { q = b; goto done; }
+    if (d3 >= 0.f && d4 <= d3) { w = bp; goto done; }
     const float vc = d1 * d4 - d3 * d2;
     if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) {
       const float v = __fdividef(d1, d1 - d3);
-      q = make_float3(a.x + ab.x * v, a.y + ab.y * v, a.z + ab.z * v);
+      w = make_float3(ap.x - ab.x * v, ap.y - ab.y * v, ap.z - ab.z * v);
       goto done;
     }
     const float3 cp = sub3(p, c);
     const float d5 = dot3(ab, cp), d6 = dot3(ac, cp);
-    if (d6 >= 0.f && d5 <= d6) { q = c; goto done; }
+    if (d6 >= 0.f && d5 <= d6) { w = cp; goto done; }
     const float vb = d5 * d2 - d1 * d6;
     if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) {
-      const float w = __fdividef(d2, d2 - d6);
-      q = make_float3(a.x + ac.x * w, a.y + ac.y * w, a.z + ac.z * w);
+      const float t = __fdividef(d2, d2 - d6);
+      w = make_float3(ap.x - ac.x * t, ap.y - ac.y * t, ap.z - ac.z * t);
       goto done;
     }
     const float va = d3 * d6 - d5 * d4;
     if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
-      const float w = __fdividef(d4 - d3, (d4 - d3) + (d5 - d6));
-      q = make_float3(b.x + (c.x - b.x) * w, b.y + (c.y - b.y) * w, b.z + (c.z - b.z) * w);
+      const float t = __fdividef(d4 - d3, (d4 - d3) + (d5 - d6));
+      w = make_float3(bp.x - (c.x - b.x) * t, bp.y - (c.y - b.y) * t, bp.z - (c.z - b.z) * t);
       goto done;
     }
     const float den = __fdividef(1.f, va + vb + vc);
-    const float v = vb * den, w = vc * den;
-    q = make_float3(a.x + ab.x * v + ac.x * w, a.y + ab.y * v + ac.y * w, a.z + ab.z * v + ac.z * w);
+    const float v = clamp01f(vb * den), t = fminf(clamp01f(vc * den), 1.f - v);
+    w = make_float3(ap.x - (ab.x * v + ac.x * t), ap.y - (ab.y * v + ac.y * t), ap.z - (ab.z * v + ac.z * t));
   }
 done:
-  const float3 dd = sub3(p, q);
-  return dot3(dd, dd);
+  return dot3(w, w);
 }
 
 // squared distance of two separated triangles: 9 edge-edge + 6 vertex-face.
