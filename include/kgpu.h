@@ -352,7 +352,8 @@ kgpu_status kgpu_self_pair_distances(kgpu_world world, int32_t robot, const floa
  * kernel.  Replaces geometry_ad.MinDistance + pytorch.ADModule backward
  * (Python/klampt/math/autodiff/geometry_ad.py:613-814,
  * Python/klampt/math/autodiff/pytorch.py:72-115).  q: [T*W*num_links],
- * L: [T], dLdq: [T*W*num_links] (may be NULL). */
+ * L: [T], dLdq: [T*W*num_links] (may be NULL).  T*W is at most 2^31 - 8193
+ * (KGPU_ERR_INVALID otherwise). */
 kgpu_status kgpu_softmin_grad(kgpu_world world, int32_t robot, const float* q, int32_t T,
                               int32_t W, double tau, double* L, float* dLdq, kgpu_stream stream);
 

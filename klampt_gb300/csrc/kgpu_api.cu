@@ -1095,6 +1095,10 @@ kgpu_status kgpu_softmin_grad(kgpu_world w, int32_t robot, const float* q, int32
   kgpu_status st = check_world(w, robot);
   if (st) return st;
   if (T < 0 || Wn < 1 || (T > 0 && (!q || !L))) return fail(KGPU_ERR_INVALID, "bad buffers");
+  // (the launches count waypoints, and chunks of them, in 32 bits)
+  if ((int64_t)T * Wn > INT32_MAX - kSoftChunk)
+    return fail(KGPU_ERR_INVALID, "T * W = %lld waypoints, at most %d a call", (long long)T * Wn,
+                INT32_MAX - kSoftChunk);
   if (!(tau > 0)) return fail(KGPU_ERR_INVALID, "tau must be positive");
   if (!w->env) return fail(KGPU_ERR_EMPTY, "distance query without an environment (robotsim.cpp:1786-1787)");
   const int nl = w->robots[robot]->nlinks;

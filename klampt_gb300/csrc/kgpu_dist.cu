@@ -782,7 +782,6 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
 // A waypoint whose pairs do not fit (list or segment table full) is flagged
 // and done by one warp in k_dist<1> / k_dist<2>.
 constexpr int kSoftSegs = 128;        // list segments per waypoint (of up to kDPairs pairs)
-constexpr int kSoftChunk = 8192;      // waypoints per chunk
 constexpr int kSoftPerWaypoint = 256; // list capacity per waypoint of a chunk, on average
 
 struct SoftArgs {

@@ -346,6 +346,7 @@ cudaError_t launch_distance(const KWorldDev* Wd, const Scratch& S, int robot, co
 cudaError_t launch_self_distance(const KWorldDev* Wd, int robot, const float* q, int B, double cutoff, double* d,
                                  int* pair, double* cp, float* grad, double* dpair, int all_pairs, int num_sms,
                                  cudaStream_t s);
+constexpr int kSoftChunk = 8192;  // waypoints per chunk of a soft-min
 // work: softmin_work_bytes() of device scratch
 size_t softmin_work_bytes(int T, int Wn, int nl, int nobj);
 cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int T,
