@@ -715,11 +715,11 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
         if (lane == 0 && bl >= 0) atomicMin(A.mkey + b / A.W, double_key(best));
       } else if (lane == 0) {
         A.d[b] = bl >= 0 ? best : A.cutoff;
-        A.pair[2 * b] = bl;
-        A.pair[2 * b + 1] = bo;
+        A.pair[2 * (size_t)b] = bl;
+        A.pair[2 * (size_t)b + 1] = bo;
         for (int i = 0; i < 3; ++i) {
-          A.cp[6 * b + i] = bl >= 0 ? bp.cp[i] : 0.0;
-          A.cp[6 * b + 3 + i] = bl >= 0 ? bp.cq[i] : 0.0;
+          A.cp[6 * (size_t)b + i] = bl >= 0 ? bp.cp[i] : 0.0;
+          A.cp[6 * (size_t)b + 3 + i] = bl >= 0 ? bp.cq[i] : 0.0;
         }
       }
       if (MODE == 0 && A.grad) {
