@@ -353,7 +353,10 @@ kgpu_status kgpu_self_pair_distances(kgpu_world world, int32_t robot, const floa
  * (Python/klampt/math/autodiff/geometry_ad.py:613-814,
  * Python/klampt/math/autodiff/pytorch.py:72-115).  q: [T*W*num_links],
  * L: [T], dLdq: [T*W*num_links] (may be NULL).  T*W is at most 2^31 - 8193
- * (KGPU_ERR_INVALID otherwise). */
+ * (KGPU_ERR_INVALID otherwise).  The world keeps device scratch between calls,
+ * 8 bytes per waypoint and the pair list of a chunk: 130 MB from 8,192
+ * waypoints on, less for fewer, or for smaller chunks when the device has not
+ * that much left. */
 kgpu_status kgpu_softmin_grad(kgpu_world world, int32_t robot, const float* q, int32_t T,
                               int32_t W, double tau, double* L, float* dLdq, kgpu_stream stream);
 

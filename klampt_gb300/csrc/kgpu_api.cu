@@ -1102,15 +1102,24 @@ kgpu_status kgpu_softmin_grad(kgpu_world w, int32_t robot, const float* q, int32
   if (!(tau > 0)) return fail(KGPU_ERR_INVALID, "tau must be positive");
   if (!w->env) return fail(KGPU_ERR_EMPTY, "distance query without an environment (robotsim.cpp:1786-1787)");
   const int nl = w->robots[robot]->nlinks;
-  const size_t need = softmin_work_bytes(T, Wn, nl, w->env->nobj);
+  const int nobj = w->env->nobj;
+  int level = 0;
+  size_t need = softmin_work_bytes(T, Wn, nl, nobj, level);
   if (need > w->scratch.dist_work_cap) {
     dfree(w->scratch.dist_work);
     w->scratch.dist_work_cap = 0;
-    CK(cudaMalloc(&w->scratch.dist_work, need));
+    // up to 130 MB for a chunk: smaller chunks where memory is short
+    cudaError_t e = cudaMalloc(&w->scratch.dist_work, need);
+    while (e == cudaErrorMemoryAllocation && level + 1 < kSoftLevels) {
+      cudaGetLastError();
+      need = softmin_work_bytes(T, Wn, nl, nobj, ++level);
+      e = cudaMalloc(&w->scratch.dist_work, need);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "kgpu_softmin_grad: scratch");
     w->scratch.dist_work_cap = need;
   }
-  return launch_status(launch_softmin(w->d_dev, w->scratch, robot, q, T, Wn, tau, L, dLdq, nl, w->env->nobj,
-                                      w->scratch.dist_work, w->num_sms, (cudaStream_t)s),
+  return launch_status(launch_softmin(w->d_dev, w->scratch, robot, q, T, Wn, tau, L, dLdq, nl, nobj,
+                                      w->scratch.dist_work, level, w->num_sms, (cudaStream_t)s),
                        "kgpu_softmin_grad");
 }
 

@@ -37,6 +37,7 @@
 //     (prismatic), with u = dd/dp at the link feature point p, accumulated as
 //     per-link force/moment sums and pulled back through the chain once per
 //     configuration (the adjoint of FK), on FP32 transforms.
+#include <algorithm>
 #include <cstddef>
 #include <cfloat>
 #include <climits>
@@ -1458,13 +1459,14 @@ struct SoftLayout {
   size_t T, delta, T64, seg, nseg, ub, mkey, item, lb, d, p, u, wsum, count, bytes;
 };
 
-SoftLayout soft_layout(int T, int Wn, int nl, int nobj)
+// level k: chunks and the smallest list 2^k times smaller (8 waypoints at the last)
+SoftLayout soft_layout(int T, int Wn, int nl, int nobj, int level)
 {
   SoftLayout L;
   const size_t B = (size_t)T * Wn;
-  L.chunk = (int)(B < (size_t)kSoftChunk ? B : (size_t)kSoftChunk);
+  L.chunk = (int)std::min(B, (size_t)(kSoftChunk >> level));
   const size_t all = (size_t)L.chunk * nl * nobj, most = (size_t)L.chunk * kSoftPerWaypoint;
-  const size_t cap = all < most ? all : (most > 65536 ? most : (all < 65536 ? all : 65536));
+  const size_t cap = std::min(all, std::max(most, (size_t)65536 >> level));
   L.cap = (int)cap;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -1492,16 +1494,19 @@ SoftLayout soft_layout(int T, int Wn, int nl, int nobj)
 
 }  // namespace
 
-size_t softmin_work_bytes(int T, int Wn, int nl, int nobj) { return soft_layout(T, Wn, nl, nobj).bytes; }
+size_t softmin_work_bytes(int T, int Wn, int nl, int nobj, int level)
+{
+  return soft_layout(T, Wn, nl, nobj, level).bytes;
+}
 
 cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int T, int Wn,
-                           double tau, double* L, float* dLdq, int nl, int nobj, void* work, int num_sms,
+                           double tau, double* L, float* dLdq, int nl, int nobj, void* work, int level, int num_sms,
                            cudaStream_t s)
 {
   if (T <= 0) return cudaSuccess;
   const size_t smem = sizeof(DistSmem) * kDW;
   const int B = T * Wn;
-  const SoftLayout lay = soft_layout(T, Wn, nl, nobj);
+  const SoftLayout lay = soft_layout(T, Wn, nl, nobj, level);
   char* w = (char*)work;
   SoftArgs A = {};
   A.robot = robot;

@@ -347,9 +347,11 @@ cudaError_t launch_self_distance(const KWorldDev* Wd, int robot, const float* q,
                                  int* pair, double* cp, float* grad, double* dpair, int all_pairs, int num_sms,
                                  cudaStream_t s);
 constexpr int kSoftChunk = 8192;  // waypoints per chunk of a soft-min
-// work: softmin_work_bytes() of device scratch
-size_t softmin_work_bytes(int T, int Wn, int nl, int nobj);
+constexpr int kSoftLevels = 11;   // chunk sizes to choose from, each half the one before
+// work: softmin_work_bytes() of device scratch; level: the chunk size, 0 the
+// largest (the results are the same)
+size_t softmin_work_bytes(int T, int Wn, int nl, int nobj, int level);
 cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, const float* q, int T,
                            int Wn, double tau, double* L, float* dLdq, int nl, int nobj, void* work,
-                           int num_sms, cudaStream_t s);
+                           int level, int num_sms, cudaStream_t s);
 }  // namespace kgpu
