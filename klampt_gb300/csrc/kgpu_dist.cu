@@ -87,6 +87,7 @@ struct DistArgs {
   // soft-min (modes 1 and 2): waypoints first .. first + B whose nseg is -1
   // (their pairs did not fit the list), see SoftArgs
   const int* nseg;
+  const float *T, *delta;    // FP32 transforms of the chunk
   int first;
   unsigned long long* mkey;  // [T] trajectory minima (double_key)
   double* wsum;        // mode 2: [waypoints] sums
@@ -498,18 +499,39 @@ __device__ int gather_objects(DistSmem& S, const KWorldDev* __restrict__ W, cons
   return count;
 }
 
+// The sums of a gradient, with their roundings spelled out: a soft-min waypoint
+// goes through k_soft_reduce or, when its pairs do not fit the list, through
+// k_dist<2>; which of the two can depend on the scheduling, and the compiler
+// need not fuse the products of two kernels alike.
+__device__ __forceinline__ float diff_products(float a, float b, float c, float d)
+{
+  return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
+__device__ __forceinline__ float dot_rn(float ax, float ay, float az, float bx, float by, float bz)
+{
+  return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
+}
+
+// Adds the weighted direction u = wgt * d at point p to a link's force and
+// moment sums.
+__device__ __forceinline__ void wrench_sum(float* F, float* M, float wgt, float dx, float dy, float dz, float px,
+                                           float py, float pz)
+{
+  const float ux = __fmul_rn(wgt, dx), uy = __fmul_rn(wgt, dy), uz = __fmul_rn(wgt, dz);
+  F[0] = __fadd_rn(F[0], ux);
+  F[1] = __fadd_rn(F[1], uy);
+  F[2] = __fadd_rn(F[2], uz);
+  M[0] = __fadd_rn(M[0], diff_products(py, uz, pz, uy));
+  M[1] = __fadd_rn(M[1], diff_products(pz, ux, px, uz));
+  M[2] = __fadd_rn(M[2], diff_products(px, uy, py, ux));
+}
+
 // Adds a pair's contribution (weight wgt, feature point p, direction u) to
 // the per-link force / moment accumulators.
 __device__ __forceinline__ void add_wrench(DistSmem& S, int lane, int l, float wgt, const PairOut& po)
 {
-  if (lane == 0) {
-    const float ux = wgt * po.dir[0], uy = wgt * po.dir[1], uz = wgt * po.dir[2];
-    const float px = (float)po.cp[0], py = (float)po.cp[1], pz = (float)po.cp[2];
-    S.F[l][0] += ux; S.F[l][1] += uy; S.F[l][2] += uz;
-    S.M[l][0] += py * uz - pz * uy;
-    S.M[l][1] += pz * ux - px * uz;
-    S.M[l][2] += px * uy - py * ux;
-  }
+  if (lane == 0)
+    wrench_sum(S.F[l], S.M[l], wgt, po.dir[0], po.dir[1], po.dir[2], (float)po.cp[0], (float)po.cp[1], (float)po.cp[2]);
   __syncwarp();
 }
 
@@ -532,20 +554,21 @@ __device__ void pullback(DistSmem& S, const KRobotDev& R, int lane, float* g_out
   __syncwarp();
   if (lane < nl && g_out) {
     const float* T = S.T[lane];
-    const float wx = T[0] * R.axis[lane][0] + T[1] * R.axis[lane][1] + T[2] * R.axis[lane][2];
-    const float wy = T[3] * R.axis[lane][0] + T[4] * R.axis[lane][1] + T[5] * R.axis[lane][2];
-    const float wz = T[6] * R.axis[lane][0] + T[7] * R.axis[lane][1] + T[8] * R.axis[lane][2];
+    const float* a = R.axis[lane];
+    const float wx = dot_rn(T[0], T[1], T[2], a[0], a[1], a[2]);
+    const float wy = dot_rn(T[3], T[4], T[5], a[0], a[1], a[2]);
+    const float wz = dot_rn(T[6], T[7], T[8], a[0], a[1], a[2]);
     float g = 0.f;
     if (R.jtype[lane] == KX_JOINT_REVOLUTE) {
       const float ox = T[9], oy = T[10], oz = T[11];
       const float* F = S.F[lane];
       const float* M = S.M[lane];
-      const float tx = M[0] - (oy * F[2] - oz * F[1]);
-      const float ty = M[1] - (oz * F[0] - ox * F[2]);
-      const float tz = M[2] - (ox * F[1] - oy * F[0]);
-      g = wx * tx + wy * ty + wz * tz;
+      const float tx = __fsub_rn(M[0], diff_products(oy, F[2], oz, F[1]));
+      const float ty = __fsub_rn(M[1], diff_products(oz, F[0], ox, F[2]));
+      const float tz = __fsub_rn(M[2], diff_products(ox, F[1], oy, F[0]));
+      g = dot_rn(wx, wy, wz, tx, ty, tz);
     } else if (R.jtype[lane] == KX_JOINT_PRISMATIC) {
-      g = wx * S.F[lane][0] + wy * S.F[lane][1] + wz * S.F[lane][2];
+      g = dot_rn(wx, wy, wz, S.F[lane][0], S.F[lane][1], S.F[lane][2]);
     }
     g_out[lane] = g;
   }
@@ -608,7 +631,13 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
       continue;
     }
     float P[12], delta;
-    warp_fk32(R, lane, q, 0.f, P, &delta);
+    if (MODE == 0) {
+      warp_fk32(R, lane, q, 0.f, P, &delta);
+    } else if (lane < nl) {  // the chunk's, so that both ways of a waypoint see the same
+      const size_t at = (size_t)it * nl + lane;
+      for (int i = 0; i < 12; ++i) P[i] = __ldg(A.T + at * 12 + i);
+      delta = __ldg(A.delta + at);
+    }
     if (lane < nl) {
       for (int i = 0; i < 12; ++i) S.T[lane][i] = P[i];
       S.delta[lane] = delta;
@@ -1070,17 +1099,11 @@ __global__ void __launch_bounds__(kDW * 32) k_soft_reduce(const KWorldDev* __res
         todo &= todo - 1;
         const double es = __shfl_sync(0xffffffffu, e, src);
         sum += es;
-        const float wgt = (float)es;
-        const float ux = wgt * __shfl_sync(0xffffffffu, u.x, src), uy = wgt * __shfl_sync(0xffffffffu, u.y, src),
-                    uz = wgt * __shfl_sync(0xffffffffu, u.z, src);
+        const float dx = __shfl_sync(0xffffffffu, u.x, src), dy = __shfl_sync(0xffffffffu, u.y, src),
+                    dz = __shfl_sync(0xffffffffu, u.z, src);
         const float px = __shfl_sync(0xffffffffu, p.x, src), py = __shfl_sync(0xffffffffu, p.y, src),
                     pz = __shfl_sync(0xffffffffu, p.z, src);
-        if (__shfl_sync(0xffffffffu, l, src) == lane) {
-          F[0] += ux; F[1] += uy; F[2] += uz;
-          M[0] += py * uz - pz * uy;
-          M[1] += pz * ux - px * uz;
-          M[2] += px * uy - py * ux;
-        }
+        if (__shfl_sync(0xffffffffu, l, src) == lane) wrench_sum(F, M, (float)es, dx, dy, dz, px, py, pz);
       }
     }
   }
@@ -1539,6 +1562,8 @@ cudaError_t launch_softmin(const KWorldDev* Wd, const Scratch& S, int robot, con
   D.scratch = S.spill;
   D.scratch_per_warp = (int)S.spill_per_warp;
   D.nseg = A.nseg;
+  D.T = A.T;
+  D.delta = A.delta;
   D.mkey = A.mkey;
   D.wsum = A.wsum;
   D.W = Wn;
