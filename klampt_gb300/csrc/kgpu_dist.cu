@@ -948,6 +948,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_soft_bound(const KWorldDev* __r
       if (lane == 0 && b < ub) atomicMin(A.ub + t, __float_as_uint(b));
     }
   }
+  count_pairs(W, cnt, lane);
 }
 
 // PASS 1: pairs within the bound of the trajectory's minimum; 2: within m + 30 tau

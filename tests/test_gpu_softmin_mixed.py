@@ -83,3 +83,17 @@ def test_one_waypoint_too_dense(built):
     assert abs(L[4] - L_o[0]) <= 1e-12 * max(1.0, abs(L_o[0]))
     assert np.abs(G[4] - G_o[0]).max() <= 1e-4 * np.abs(G_o[0]).max() + 1e-7
     w.close()
+
+
+def test_counters_include_the_bounding_evaluations(built):
+    """One link, one object too large for a vertex-pair bound: evaluated for
+    the bound, for the minimum and for the sum."""
+    from klampt_gb300.engine import World
+    rng = np.random.default_rng(1)
+    H = sc.terrain_heights(60, 50, 0.04, rng)
+    env = sc.env_from_objects("terrain", [sc.heightfield_mesh(60, 50, 0.04, H, (-1.2, -1.0, -1.2))])
+    robot = sc.arm(1, rings=2, segments=8)
+    w = World(env, [robot])
+    L, _, pairs = _run(w, np.zeros((1, 1, 1), np.float32), 0.01)
+    w.close()
+    assert np.isfinite(L).all() and pairs == 3
