@@ -60,9 +60,7 @@ struct __align__(16) DistSmem {
   float T[kMaxLinks][12];
   float delta[kMaxLinks];
   double q64[kMaxLinks];
-  const float* item_qa;
-  const float* item_qb;
-  int item_k, item_n;
+  const float* item_q;
   // ... and what gathering the pairs and the gradient need besides: kernels
   // that only evaluate pairs leave it out (kEvalSmem), and the L1 gains it
   // (soft-min over 6,400 waypoints: 3%)
@@ -75,7 +73,6 @@ struct __align__(16) DistSmem {
 constexpr size_t kEvalSmem = offsetof(DistSmem, gstack);
 
 struct DistArgs {
-  int mode;            // 0 min distance, 1 soft-min pass 1 (minimum), 2 soft-min pass 2
   int robot;
   const float* q;      // [B, L]
   int B;
@@ -119,16 +116,10 @@ struct DCnt {
   PairCnt p;  // per lane
 };
 
-__device__ __forceinline__ double item_q64(const DistSmem& S, int lane)
-{
-  if (S.item_qb == nullptr) return (double)S.item_qa[lane];
-  return kx_interp((double)S.item_qa[lane], (double)S.item_qb[lane], S.item_k, S.item_n);
-}
-
 __device__ __noinline__ void dist_fk64(DistSmem& S, const KRobotDev& R, double (*T64)[12], int lane, int& fk64)
 {
   if (fk64) return;
-  if (lane < R.nlinks) S.q64[lane] = item_q64(S, lane);
+  if (lane < R.nlinks) S.q64[lane] = (double)S.item_q[lane];
   __syncwarp();
   warp_fk64(R, S.q64, T64, lane);
   fk64 = 1;
@@ -594,7 +585,7 @@ __device__ __forceinline__ void count_pairs(const KWorldDev* __restrict__ W, con
   }
 }
 
-// MODE (A.mode): 0 minimum distance with closest points and gradient; 1 and
+// MODE: 0 minimum distance with closest points and gradient; 1 and
 // 2 the soft-min's two passes (trajectory minima, every pair below m + K tau)
 // for the waypoints whose pairs did not fit the soft-min's list; one
 // instantiation each, so that a launch carries only its mode's code
@@ -618,12 +609,7 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     if (it >= (unsigned)A.B) break;
     const int b = MODE == 0 ? (int)it : A.first + (int)it;
     if (MODE != 0 && A.nseg[it] >= 0) continue;
-    if (lane == 0) {
-      S.item_qa = A.q + (size_t)b * nl;
-      S.item_qb = nullptr;
-      S.item_k = 0;
-      S.item_n = 0;
-    }
+    if (lane == 0) S.item_q = A.q + (size_t)b * nl;
     float q = lane < nl ? __ldg(A.q + (size_t)b * nl + lane) : 0.f;
     __syncwarp();
     if (__any_sync(0xffffffffu, lane < nl && !(fabsf(q) < 1.0e6f))) {
@@ -1161,10 +1147,6 @@ __global__ void k_softmin_final(const double* wsum, const unsigned long long* mk
 // triangle pairs within the error band finalised in canonical FP64.
 constexpr int kSW = 2;  // warps per block of k_self_dist
 
-struct __align__(16) SelfDistSmem;
-__device__ __noinline__ float link_pair_seed(SelfDistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
-                                             int lane, int i, int j);
-
 struct __align__(16) SelfDistSmem {
   float T[kMaxLinks][12];
   float delta[kMaxLinks];
@@ -1459,7 +1441,6 @@ cudaError_t launch_distance(const KWorldDev* Wd, const Scratch& S, int robot, co
   cudaError_t e = cudaMemsetAsync(S.counters + 8, 0, sizeof(unsigned int), s);
   if (e != cudaSuccess) return e;
   DistArgs A = {};
-  A.mode = 0;
   A.robot = robot;
   A.q = q;
   A.B = B;
