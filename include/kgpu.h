@@ -166,7 +166,8 @@ kgpu_status kgpu_world_enable_self_pair(kgpu_world world, int32_t robot, int32_t
 /* Named options: "eps_extra" (m, additional inflation of every FP32 test on
  * top of the computed error bounds, default 0), "blocks_per_sm" (2, 3 or 4
  * resident engine blocks per SM), "grab" (work items per queue atomic, 1..16),
- * "job_flush" (triangle-pair jobs batched before testing, 8..64),
+ * "job_flush" (triangle-pair jobs batched before testing, 8..64; until it is
+ * set 64, or 32 in batches of fewer work items than resident warps),
  * "edge_chunk" (consecutive steps of an edge per work item, 1..64, default
  * 16; the item checks them in groups of 32 / L steps, L the robot's link
  * count rounded up to 8, 16 or 32, earliest step first), "fp64_inline" (1: triangle pairs the FP32 tests

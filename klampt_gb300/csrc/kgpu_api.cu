@@ -855,7 +855,7 @@ kgpu_status kgpu_world_get_option(kgpu_world w, const char* name, double* v)
   else if (!strcmp(name, "warps_per_block")) *v = engine_warps_per_block();
   else if (!strcmp(name, "blocks_per_sm")) *v = w->blocks_per_sm;
   else if (!strcmp(name, "grab")) *v = w->grab;
-  else if (!strcmp(name, "job_flush")) *v = w->job_flush;
+  else if (!strcmp(name, "job_flush")) *v = w->job_flush ? w->job_flush : 64;
   else if (!strcmp(name, "edge_chunk")) *v = w->edge_chunk;
   else if (!strcmp(name, "fp64_inline")) *v = w->fp64_inline;
   else if (!strcmp(name, "num_sms")) *v = w->num_sms;

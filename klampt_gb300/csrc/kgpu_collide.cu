@@ -707,9 +707,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
   // 231 us, 8 edges 211 -> 183 us
   const bool deal = (unsigned)total <= gridDim.x * (unsigned)kWarps;
   bool dealt = false;
-  // jobs tested earlier: a contact found sooner ends the item, and lanes are
-  // idle anyway (500 feasibility checks 247 -> 241 us, 24 edges 231 -> 217 us)
-  const int job_flush = deal ? min(job_flush_opt, 32) : job_flush_opt;
+  // jobs tested earlier, unless the option is set: a contact found sooner ends
+  // the item, and lanes are idle anyway (500 feasibility checks 247 -> 241 us,
+  // 24 edges 231 -> 217 us)
+  const int job_flush = deal && A.job_flush == 0 ? 32 : job_flush_opt;
 
 #pragma unroll 1
   for (;;) {

@@ -255,7 +255,7 @@ struct kgpu_world_s {
   double eps_extra = 0.0;
   int blocks_per_sm = 3;   // resident 8-warp engine blocks per SM (2, 3 or 4)
   int grab = 2;            // work items per queue atomic (1..16)
-  int job_flush = 64;      // triangle-pair jobs collected before testing them (8..64)
+  int job_flush = 0;       // triangle-pair jobs collected before testing them (8..64); 0: not set
   int edge_chunk = 16;     // consecutive steps of an edge per work item (1..64)
   int fp64_inline = -1;    // FP64 triangle tests inline (1) or deferred to k_band (0); -1: deferred
   // caps below the allocated scratch (0 = none): the undecided-pair list and
