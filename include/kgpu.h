@@ -165,7 +165,8 @@ kgpu_status kgpu_world_enable_self_pair(kgpu_world world, int32_t robot, int32_t
 
 /* Named options: "eps_extra" (m, additional inflation of every FP32 test on
  * top of the computed error bounds, default 0), "blocks_per_sm" (2, 3 or 4
- * resident engine blocks per SM), "grab" (work items per queue atomic, 1..16),
+ * resident engine blocks per SM; until it is set 3, or 2 for at most 512
+ * edges), "grab" (work items per queue atomic, 1..16),
  * "job_flush" (triangle-pair jobs batched before testing, 8..64; until it is
  * set 64, or 32 in batches of fewer work items than resident warps),
  * "edge_chunk" (consecutive steps of an edge per work item, 1..64, default

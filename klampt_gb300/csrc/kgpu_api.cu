@@ -244,6 +244,7 @@ Scratch engine_scratch(kgpu_world w, Scratch S)
   const size_t spill = (size_t)w->spill_cap_opt + (size_t)engine_scratch_doubles();
   if (w->spill_cap_opt > 0 && spill < S.spill_per_warp) S.spill_per_warp = spill;
   S.stage_nodes = w->stage_nodes;
+  S.small_kernel = !w->blocks_set || w->blocks_per_sm == 2;
   return S;
 }
 }  // namespace kgpu
@@ -806,6 +807,7 @@ kgpu_status kgpu_world_set_option(kgpu_world w, const char* name, double v)
     int k = (int)v;
     if (k < 2 || k > 4) return fail(KGPU_ERR_INVALID, "blocks_per_sm must be 2, 3 or 4");
     w->blocks_per_sm = k;
+    w->blocks_set = true;
   } else if (!strcmp(name, "grab")) {
     int k = (int)v;
     if (k < 1 || k > 16) return fail(KGPU_ERR_INVALID, "grab must be in [1,16]");

@@ -1671,9 +1671,10 @@ cudaError_t dispatch_engine(const KWorldDev* W, EngineArgs A, const Scratch& S, 
     return err;
   if (A.inline64) return per_sm == 3 ? launch_engine<3, true>(W, A, blocks, s) : launch_engine<2, true>(W, A, blocks, s);
   const int sms = per_sm > 0 && blocks / per_sm > 0 ? blocks / per_sm : 1;
-  // few edges: the SMALL kernel, with the registers of 2 blocks per SM whatever
-  // the option (there are warps to spare); 1,500 edges are no faster with it
-  const bool small = A.mode == MODE_EDGES && A.stage_nodes == 0 && A.E <= kSmallEdges;
+  // few edges: the SMALL kernel, with the registers of 2 blocks per SM (there
+  // are warps to spare), unless the caller set another residency; 1,500 edges
+  // are no faster with it
+  const bool small = A.mode == MODE_EDGES && A.stage_nodes == 0 && S.small_kernel && A.E <= kSmallEdges;
   switch (small ? 0 : per_sm) {
     case 0:
       k_engine<2, false, true, false, true><<<2 * sms, kWarps * 32, engine_smem<false>(), s>>>(W, A);

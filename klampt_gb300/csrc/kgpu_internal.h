@@ -171,6 +171,8 @@ struct Scratch {
   // launch setting carried with the scratch: environment nodes a staged
   // engine block copies to shared memory (0: the unstaged kernels)
   int stage_nodes = 0;
+  // few edges may take the SMALL kernel, which has 2 blocks per SM
+  bool small_kernel = true;
   // edge plans: events recorded (as graph nodes) around the main pass, so
   // that its own device time can be read after a launch
   cudaEvent_t main_pass_ev[2] = {nullptr, nullptr};
@@ -254,6 +256,7 @@ struct kgpu_world_s {
   double eps_env = 0.0;
   double eps_extra = 0.0;
   int blocks_per_sm = 3;   // resident 8-warp engine blocks per SM (2, 3 or 4)
+  bool blocks_set = false; // set by the caller: holds for few edges too
   int grab = 2;            // work items per queue atomic (1..16)
   int job_flush = 0;       // triangle-pair jobs collected before testing them (8..64); 0: not set
   int edge_chunk = 16;     // consecutive steps of an edge per work item (1..64)
