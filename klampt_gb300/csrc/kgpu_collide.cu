@@ -645,11 +645,11 @@ __device__ __noinline__ unsigned traverse(WarpSmem& S, const KWorldDev* __restri
 // pairs are common and an inline FP64 contact ends an item early) or as the
 // fallback after a main pass whose list overflowed (otherwise it returns at
 // once); its verdicts overwrite the main pass's.
-// SMALL (edges): batches of few edges, whose steps are in work side by side;
-// those after an edge's first contact stop when it is known.  An instantiation
-// of its own, because the check costs large batches 3% by its mere presence
-// (16,384 edges 1,620 -> 1,672 us).  24 edges 231 -> 176 us, 60 edges 272 ->
-// 208 us, 200 edges 194 -> 173 us.
+// SMALL (edges): few edges, many of whose steps are in work side by side (all of
+// them, one per warp, while there are fewer than warps); those after an edge's
+// first contact stop when it is known.  An instantiation of its own, because
+// the check costs large batches 3% by its mere presence (16,384 edges 1,620 ->
+// 1,672 us).
 template <int MINB, bool FP64, bool EDGES, bool STAGE = false, bool SMALL = false>
 __global__ void __launch_bounds__(kWarps * 32, MINB)
     k_engine(const KWorldDev* __restrict__ W, const EngineArgs A)
@@ -1672,8 +1672,12 @@ cudaError_t dispatch_engine(const KWorldDev* W, EngineArgs A, const Scratch& S, 
   if (A.inline64) return per_sm == 3 ? launch_engine<3, true>(W, A, blocks, s) : launch_engine<2, true>(W, A, blocks, s);
   const int sms = per_sm > 0 && blocks / per_sm > 0 ? blocks / per_sm : 1;
   // few edges: the SMALL kernel, with the registers of 2 blocks per SM (there
-  // are warps to spare), unless the caller set another residency; 1,500 edges
-  // are no faster with it
+  // are warps to spare), unless the caller set another residency.  Calls with
+  // the default options, means over six batches, common kernel -> SMALL: 24
+  // edges of up to 400 steps 253 -> 192 us, 100 361 -> 283, 256 500 -> 389, 512
+  // 516 -> 413, 1,000 578 -> 455, 2,500 700 -> 576; of up to 30 steps 24 205 ->
+  // 180, 256 252 -> 272, 512 385 -> 298.  The line is below where it would pay
+  // (16,384 edges lose 3%; not measured between 2,500 and those)
   const bool small = A.mode == MODE_EDGES && A.stage_nodes == 0 && S.small_kernel && A.E <= kSmallEdges;
   switch (small ? 0 : per_sm) {
     case 0:
