@@ -60,7 +60,9 @@ struct __align__(16) DistSmem {
   float T[kMaxLinks][12];
   float delta[kMaxLinks];
   double q64[kMaxLinks];
-  const float* item_q;
+  const float* item_qa;
+  const float* item_qb;
+  int item_k, item_n;
   // ... and what gathering the pairs and the gradient need besides: kernels
   // that only evaluate pairs leave it out (kEvalSmem), and the L1 gains it
   // (soft-min over 6,400 waypoints: 3%)
@@ -116,10 +118,20 @@ struct DCnt {
   PairCnt p;  // per lane
 };
 
+// (No distance kernel sets an edge's second end.  Without this branch, the
+// soft-min takes 40.4 instead of 39.4 ms over 6,400 waypoints, the same with the
+// shared memory's layout kept: its kernels are bound by fetching their code, and
+// this moves it.)
+__device__ __forceinline__ double item_q64(const DistSmem& S, int lane)
+{
+  if (S.item_qb == nullptr) return (double)S.item_qa[lane];
+  return kx_interp((double)S.item_qa[lane], (double)S.item_qb[lane], S.item_k, S.item_n);
+}
+
 __device__ __noinline__ void dist_fk64(DistSmem& S, const KRobotDev& R, double (*T64)[12], int lane, int& fk64)
 {
   if (fk64) return;
-  if (lane < R.nlinks) S.q64[lane] = (double)S.item_q[lane];
+  if (lane < R.nlinks) S.q64[lane] = item_q64(S, lane);
   __syncwarp();
   warp_fk64(R, S.q64, T64, lane);
   fk64 = 1;
@@ -609,7 +621,12 @@ __global__ void __launch_bounds__(kDW * 32, 2) k_dist(const KWorldDev* __restric
     if (it >= (unsigned)A.B) break;
     const int b = MODE == 0 ? (int)it : A.first + (int)it;
     if (MODE != 0 && A.nseg[it] >= 0) continue;
-    if (lane == 0) S.item_q = A.q + (size_t)b * nl;
+    if (lane == 0) {
+      S.item_qa = A.q + (size_t)b * nl;
+      S.item_qb = nullptr;
+      S.item_k = 0;
+      S.item_n = 0;
+    }
     float q = lane < nl ? __ldg(A.q + (size_t)b * nl + lane) : 0.f;
     __syncwarp();
     if (__any_sync(0xffffffffu, lane < nl && !(fabsf(q) < 1.0e6f))) {
