@@ -319,7 +319,10 @@ kgpu_status kgpu_check_edges_plain64_pairs(kgpu_world world, int32_t robot, cons
  * upperBound = cutoff) and WorldPlannerSettings::DistanceLowerBound
  * (PlannerSettings.cpp:372-483).  d: [B] (cutoff when nothing is closer),
  * pair: [B*2] (link, object) or (-1,-1), cp: [B*6] closest points in world
- * frame (link side, object side), grad: [B*num_links] (may be NULL). */
+ * frame (link side, object side), grad: [B*num_links] (may be NULL).  Where the
+ * surfaces meet and no link vertex is inside a convex object, d and grad are 0
+ * and both points are some vertex of a link triangle (which one is not
+ * specified). */
 kgpu_status kgpu_distance(kgpu_world world, int32_t robot, const float* q, int32_t B,
                           double cutoff, double* d, int32_t* pair, double* cp, float* grad,
                           kgpu_stream stream);

@@ -195,7 +195,7 @@ __device__ __forceinline__ float depth_band(const KNode& ob, float dd)
 // its deepest vertex in FP64) takes a few hundred thousand.  Among boxes most
 // pairs a configuration still has to look at after its first contact are
 // shallower contacts: 32,768 terrain clearances 38.9 -> 27.4 ms with this test
-// (20.7 with the later work on the pair traversal).
+// (19-21 by the drawn configurations with the later work on the pair traversal).
 __device__ __noinline__ bool may_be_deeper(const DistSmem& S, const KWorldDev* __restrict__ W, const KRobotDev& R,
                                            int lane, int l, int o, float need)
 {
@@ -1278,8 +1278,8 @@ __device__ __noinline__ void self_pairs(SelfDistSmem& S, const KWorldDev* __rest
 // (i, j) order evaluated most of a humanoid's 435.  The result is the
 // lexicographic minimum (distance, pair), whatever the order.  Blocks of two
 // warps, so that a costly configuration holds up one other at most.  8,192
-// humanoid configurations: 15.4 -> 5.96 ms by this order (5.15 ms with the
-// later work on the pair traversal).
+// humanoid configurations: 15.4 -> 5.96 ms by this order (4.3-7.5 ms by
+// the drawn postures with the later work on the pair traversal).
 __global__ void __launch_bounds__(kSW * 32, 16 / kSW) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -102,12 +102,13 @@ __device__ __noinline__ void ray_decide(const KWorldDev* __restrict__ W, const d
   }
 }
 
-// Bound by the divergent traversal (a lane's next node and triangles are L1 and
-// L2 loads it waits for).  A child's box is tested once, before it is pushed
+// Bound by the divergent traversal (7.4 of 32 lanes active; a lane's next node
+// and triangles are L1 and L2 loads, 22% of the stalls) and the FP64 pipe, 46%
+// busy with the decisions at the end.  A child's box is tested once, before it is pushed
 // (with where the ray enters it, so that a popped child beyond the best hit is
 // dropped unread), and the nearer child is entered directly.  640 x 480 camera
 // rays into 640 k triangles: 946 -> 581 us for the
-// call (node tests once instead of twice, FP64 decisions at the end of the ray).
+// call, 528 of it here (node tests once instead of twice, FP64 decisions at the end of the ray).
 __global__ void __launch_bounds__(128) k_ray(const KWorldDev* __restrict__ W, const float* __restrict__ s,
                                              const float* __restrict__ d, int R, int* obj, int* tri,
                                              double* tout, double* point)
