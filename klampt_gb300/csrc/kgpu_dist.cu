@@ -1278,7 +1278,7 @@ __device__ __noinline__ void self_pairs(SelfDistSmem& S, const KWorldDev* __rest
 // (i, j) order evaluated most of a humanoid's 435.  The result is the
 // lexicographic minimum (distance, pair), whatever the order.  Blocks of two
 // warps, so that a costly configuration holds up one other at most.  8,192
-// humanoid configurations: 15.4 -> 5.96 ms by this order (4.3-7.5 ms by
+// humanoid configurations: 15.4 -> 5.96 ms by this order (4.3-8.3 ms by
 // the drawn postures with the later work on the pair traversal).
 __global__ void __launch_bounds__(kSW * 32, 16 / kSW) k_self_dist(const KWorldDev* __restrict__ W, const SelfDistArgs A)
 {

@@ -24,7 +24,7 @@
 // a bit mask instead of a binary search and a division, and minima compared as
 // integers, the same four went from 3.9, 45.2, 5.75 and 24.7 ms to 3.5, 39.2,
 // 5.15 and 20.7 ms (mostly by the roots; the last two differ by the drawn
-// configurations, 4.3-7.5 and 19-21 ms).
+// configurations, 4.3-8.3 and 19-21 ms).
 #pragma once
 
 #include "kgpu_dist32.cuh"
